@@ -178,6 +178,13 @@ def stencil_launch_bytes(A, nvec, iters, outer, fp32, df=0):
     return u * (88 * iters + 24)
 
 
+def cheb_launch_bytes(A, nvec, steps, outer):
+    """Algorithmic bytes of a Chebyshev solve launch (csrc/cheby.cuh), per unknown: 16 B per step but the first
+    (read x_k, x_{k-1}, r; write x_{k+1}), the start 12 B (read b, write r), 20 B per true residual (read
+    x as two floats and b, write r), the FP32 check 8 B, and the solution 16 B."""
+    return A.shape[0] * nvec * (16 * max(steps - 1, 0) + 12 + 20 * outer + 8 + 16)
+
+
 # DRAM bytes (read + write) per unknown and iteration of the FP32 stencil CG, measured with ncu on a GB300
 # (dram__bytes_read.sum + dram__bytes_write.sum of a 300-iteration elastic 128^3 launch / (300 x unknowns):
 # (10.91 + 28.00) GB / 300 / 6.29 M for the current kernel); the vectors fit the L2 about half way, so this
@@ -459,6 +466,8 @@ def run_ours(args):
         if hasattr(A, "ncomp") and fp32 and L.precond == "fft" and k in FFT_SLOTS and nv == 1 and \
                 A.fft_plan() is not None:
             kn, b = "cg_stencil_fft_kernel", fft_launch_bytes(A, its, inf["outer"], warm, k in L.carry)
+        elif hasattr(A, "ncomp") and fp32 and k > 1:
+            kn, b = "cheb_stencil_kernel", cheb_launch_bytes(A, nv, its, inf["outer"])
         elif hasattr(A, "ncomp"):
             kn = "cg_stencil_ir_kernel" if fp32 else "cg_stencil_fp64_kernel"
             b = stencil_launch_bytes(A, nv, its, inf["outer"], fp32, inf["df_updates"])

@@ -16,7 +16,7 @@ _lib = None
 
 CPM_OK, CPM_NOT_CONVERGED, CPM_BARRIER_TIMEOUT, CPM_NONFINITE, CPM_BAD_ARG, CPM_CUDA_ERROR = range(6)
 # iteration forms of the FP32 stencil CG (cpm_cg_opts.form)
-CG_FORM_DEFAULT, CG_FORM_THREE_BARRIER, CG_FORM_TWO_BARRIER, CG_FORM_FFT_PCG = 0, 1, 2, 3
+CG_FORM_DEFAULT, CG_FORM_THREE_BARRIER, CG_FORM_TWO_BARRIER, CG_FORM_FFT_PCG, CG_FORM_FP64_RESIDUALS = 0, 1, 2, 3, 4
 # spectrum layouts of the FFT preconditioner (cpm_fft_precond.layout)
 FFT_LAYOUT_AUTO, FFT_LAYOUT_SLAB, FFT_LAYOUT_PASSES = 0, 1, 2
 STATUS_NAMES = {0: "ok", 1: "not converged", 2: "grid barrier timeout", 3: "non-finite value", 4: "bad argument",
@@ -88,6 +88,7 @@ _PROTOS = {
     "cpm_spmv_csr_multi": (C.c_int, [C.POINTER(CSR), vp, vp, vp, vp, dbl, C.c_int, vp, i64, vp]),
     "cpm_cg_workspace_bytes": (C.c_size_t, [i64, C.c_int, C.c_int]),
     "cpm_cg_stencil_workspace_bytes": (C.c_size_t, [i64, C.c_int, C.c_int]),
+    "cpm_cg_stencil_workspace": (C.c_size_t, [C.POINTER(Stencil), C.c_int, C.c_int]),
     "cpm_stencil_df_error_bound": (C.c_double, [C.POINTER(Stencil)]),
     "cpm_cg_solve": (C.c_int, [C.POINTER(CSR), vp, vp, C.c_int, C.POINTER(CGOpts), vp, C.c_size_t, vp, vp]),
     "cpm_cg_solve_noalloc": (C.c_int, [C.POINTER(CSR), vp, vp, C.c_int, C.POINTER(CGOpts), vp, vp]),

@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "cheby.cuh"
 #include "stencil_ops.cuh"
 
 namespace cpm {
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
 constexpr int kIRThreads = 256;
 
 template <int NC, int NR>
-__global__ void __launch_bounds__(kIRThreads, 4) cg_stencil_ir_kernel(const __grid_constant__ StencilCG a) {
+__device__ __forceinline__ void cg_stencil_ir_body(const StencilCG &a) {
   constexpr int U = NC * NR;
   constexpr int NS = n_systems<NC, NR>();
   constexpr int TH = kIRThreads;
@@ -536,6 +537,26 @@ __global__ void __launch_bounds__(kIRThreads, 4) cg_stencil_ir_kernel(const __gr
   }
 }
 
+template <int NC, int NR>
+__global__ void __launch_bounds__(kIRThreads, 4) cg_stencil_ir_kernel(const __grid_constant__ StencilCG a) {
+  cg_stencil_ir_body<NC, NR>(a);
+}
+
+// ---------------------------------------------------------------- Chebyshev iteration (csrc/cheby.cuh)
+// The default of the FP32 form for the scalar stencils that cheb_operator accepts.  A system that turns
+// out not to fit on the device (a flagged row that is not pinned, values that are not finite in floats) is
+// solved by the CG above in the same launch.
+struct ChebSolve {
+  ChebSys sys;
+  ChebOp op;
+  StencilCG cg;
+};
+
+template <int NR>
+__global__ void __launch_bounds__(kChebThreads, kChebBlocks) cheb_stencil_kernel(const __grid_constant__ ChebSolve a) {
+  __shared__ double s_red[NR + 1][kCGWarps];
+  if (!cheb_solve<NR>(a.sys, a.op, blockIdx.x, s_red)) cg_stencil_ir_body<1, NR>(a.cg);
+}
 
 // ---------------------------------------------------------------- FP32 CG with two grid barriers per iteration
 // The refinement form of cg_stencil_ir_kernel rearranged so that an iteration
@@ -906,9 +927,128 @@ static double df_error_bound(const cpm_stencil *s) {
   return 2.0 * g * s1 / smin;
 }
 
+bool cheb_operator(const double *c, int ncomp, ChebOp *op) {
+  if (ncomp != 1) return false;
+  double ev[8] = {0}, s1 = 0.0, odd = 0.0;
+  for (int d = 0; d < 27; ++d) {
+    const int m = 4 * (d / 9 != 1) + 2 * ((d / 3) % 3 != 1) + (d % 3 != 1);
+    ev[m] += c[d] / (double)((m & 4 ? 2 : 1) * (m & 2 ? 2 : 1) * (m & 1 ? 2 : 1));
+    s1 += std::fabs(c[d]);
+  }
+  for (int d = 0; d < 27; ++d)
+    odd += std::fabs(c[d] - ev[4 * (d / 9 != 1) + 2 * ((d / 3) % 3 != 1) + (d % 3 != 1)]);
+  if (!(odd <= std::ldexp(s1, -50))) return false;
+  double lo = INFINITY, hi = -INFINITY;
+  for (int m = 0; m < 8; ++m) {
+    double sig = 0.0;
+    for (int e = 0; e < 8; ++e) {
+      double w = ev[e];
+      for (int ax = 0; ax < 3; ++ax)
+        if ((e >> ax) & 1) w *= (m >> ax) & 1 ? -2.0 : 2.0;
+      sig += w;
+    }
+    lo = std::min(lo, sig);
+    hi = std::max(hi, sig);
+  }
+  if (!(lo > 0.0) || !(hi <= 64.0 * lo)) return false;
+  if (!op) return true;
+  lo *= 1.0 - 1e-6;  // the FP32 coefficients' rounding
+  hi *= 1.0 + 1e-6;
+  const double theta = 0.5 * (hi + lo), delta = std::max(0.5 * (hi - lo), 1e-3 * theta), sigma = theta / delta;
+  for (int e = 0; e < 8; ++e) {
+    op->c64[e] = ev[e];
+    op->c[e] = (float)ev[e];
+    op->cl[e] = (float)(ev[e] - (double)op->c[e]);
+  }
+  op->itheta = 1.0 / theta;
+  op->q32 = std::ldexp(11.0 * s1 / lo + 3.0, -24);
+  op->acosh_s = std::acosh(sigma);
+  double rho = 1.0 / sigma;
+  for (int k = 0; k < kChebMaxSteps; ++k) {
+    const double next = 1.0 / (2.0 * sigma - rho);
+    op->w[k] = (float)(next * rho);
+    op->g[k] = (float)(2.0 * next / delta);
+    rho = next;
+  }
+  return true;
+}
+
+int cheb_cold_steps(const ChebOp &op, double tol) {
+  int steps = 0;
+  for (double res = 1.0; res > kChebAim * tol && steps < 100000;) {
+    const int k = cheb_steps(res, kChebAim * tol, op.acosh_s);
+    steps += k;
+    res *= std::max(2.0 * std::exp(-k * op.acosh_s), 1.0 / kChebCycle);
+  }
+  return steps;
+}
+
+// Vector k of the iteration's storage (element 0 behind the pad; 32-byte aligned).
+static float *cheb_vec(float *base, const cpm_stencil *s, int nrhs, int k) {
+  const size_t f = align256(sizeof(float) * cheb_vec_floats(s->nx, s->ny, s->nz, nrhs)) / sizeof(float);
+  return base + k * f + kChebPad;
+}
+
+// Bytes in front of the solvers' vectors in a workspace.
+static size_t head_bytes() { return layout(0, 1, 1, nullptr, nullptr); }
+
+// Launch of the Chebyshev solve; *done tells whether it applies: the default form, the error bound of a
+// double-float residual (and with it of an x held as two floats) at most a quarter of the tolerance, and
+// at least four times the steps of a cold start before maxiter (nearer to it CG's smaller count may decide
+// between converged and not).
+template <int NR>
+static int launch_cheb(const cpm_stencil *s, const cpm_cg_opts *o, const StencilCG &cg, Workspace &w, float *vecs,
+                       cudaStream_t st, bool *done) {
+  *done = false;
+  ChebSolve a;
+  const double e = df_error_bound(s);
+  if (!vecs || (o->form != CPM_CG_FORM_DEFAULT && o->form != CPM_CG_FORM_FP64_RESIDUALS) ||
+      !(e > 0.0 && e <= 0.25 * o->tol) || !cheb_operator(s->coef, s->ncomp, &a.op) ||
+      o->maxiter < 4 * cheb_cold_steps(a.op, o->tol))
+    return CPM_OK;
+  a.cg = cg;
+  a.op.df = o->form == CPM_CG_FORM_DEFAULT;
+  a.op.df_err = e;
+  a.op.timeout_ns = cg.timeout_ns;
+  ChebSys &y = a.sys;
+  y = ChebSys{};
+  y.nx = s->nx;
+  y.ny = s->ny;
+  y.nz = s->nz;
+  y.n = cg.S.n;
+  y.flags = s->flags;
+  y.b = cg.b;
+  y.x = cg.x;
+  y.use_init_dev = cg.use_init_dev;
+  y.use_init_host = cg.use_init_host;
+  y.maxiter = cg.maxiter;
+  y.tol = cg.tol;
+  y.info = cg.info;
+  for (int k = 0; k < 5; ++k) y.v[k] = cheb_vec(vecs, s, NR, k);
+  y.part = w.part;
+  y.bar = w.bar;
+  const int sms = sm_count();
+  cheb_layout(y, NR, sms);
+  if ((size_t)y.half > kPartHalf) return CPM_OK;
+  int occ = 0;
+  CPM_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cheb_stencil_kernel<NR>, kChebThreads, 0));
+  if (occ < 1) return CPM_OK;
+  const int most = std::max(y.chunks, std::max(y.rchunks, y.lchunks));
+  const int G = std::min(most, std::min(occ * sms, (int)kMaxGrid));
+  y.ncta = G;
+  a.cg.dofs_per_cta = ((y.n + G - 1) / G + 31) / 32 * 32;
+  CPM_TRY(cudaMemsetAsync(w.bar, 0, sizeof(GridBarrier), st));
+  CPM_TRY(cudaMemsetAsync(cg.info, 0, sizeof(cpm_cg_info), st));
+  void *args[] = {&a};
+  CPM_TRY(cudaLaunchCooperativeKernel((const void *)cheb_stencil_kernel<NR>, dim3((unsigned)G), dim3(kChebThreads),
+                                      args, 0, st));
+  *done = true;
+  return CPM_OK;
+}
+
 template <int NC, int NR>
 static int launch_stencil_cg(const cpm_stencil *s, const double *b, double *x, const cpm_cg_opts *o, Workspace &w,
-                             float *xlo, cpm_cg_info *info, cudaStream_t st) {
+                             float *xlo, float *vecs, cpm_cg_info *info, cudaStream_t st) {
   StencilCG a{};
   a.S = to_op(s);
   a.b = b;
@@ -939,7 +1079,7 @@ static int launch_stencil_cg(const cpm_stencil *s, const double *b, double *x, c
   // x (the free pb32 vector and xlo) and an error bound at most a quarter of the tolerance, so that
   // most convergence decisions can be taken on them
   a.df_err = -1.0;
-  if (!fp64 && !two && NC == 1 && xlo) {
+  if (!fp64 && !two && NC == 1 && xlo && o->form != CPM_CG_FORM_FP64_RESIDUALS) {
     const double e = df_error_bound(s);
     if (e > 0.0 && e <= 0.25 * o->tol) {
       a.df_err = e;
@@ -949,6 +1089,14 @@ static int launch_stencil_cg(const cpm_stencil *s, const double *b, double *x, c
         const float h = (float)s->coef[d];
         a.cdf[d] = df::DF(h, (float)(s->coef[d] - (double)h));
       }
+    }
+  }
+  if constexpr (NC == 1) {
+    if (!fp64) {
+      a.quads = quads_ok(s) && ((uintptr_t)x & 15) == 0 ? 1 : 0;
+      bool done;
+      if (int err = launch_cheb<NR>(s, o, a, w, vecs, st, &done)) return err;
+      if (done) return CPM_OK;
     }
   }
   const void *fn = fp64 ? (const void *)cg_stencil_fp64_kernel<NC, NR>
@@ -1015,10 +1163,14 @@ extern "C" int cpm_cg_solve_stencil(const cpm_stencil *S, const double *b, doubl
   float *xlo = nullptr;
   if (prec && workspace_bytes >= cpm_cg_stencil_workspace_bytes(unknowns, nrhs, prec))
     xlo = (float *)((char *)workspace + need);
+  // the Chebyshev iteration's vectors take the place of the CG's where they fit
+  float *vecs = nullptr;
+  if (prec && workspace_bytes >= cpm_cg_stencil_workspace(S, nrhs, prec))
+    vecs = (float *)((char *)workspace + head_bytes());
   cudaStream_t st = (cudaStream_t)stream;
-  if (S->ncomp == 3) return launch_stencil_cg<3, 1>(S, b, x, opts, w, xlo, info_dev, st);
-  return nrhs == 1 ? launch_stencil_cg<1, 1>(S, b, x, opts, w, xlo, info_dev, st)
-                   : launch_stencil_cg<1, 3>(S, b, x, opts, w, xlo, info_dev, st);
+  if (S->ncomp == 3) return launch_stencil_cg<3, 1>(S, b, x, opts, w, xlo, vecs, info_dev, st);
+  return nrhs == 1 ? launch_stencil_cg<1, 1>(S, b, x, opts, w, xlo, vecs, info_dev, st)
+                   : launch_stencil_cg<1, 3>(S, b, x, opts, w, xlo, vecs, info_dev, st);
 }
 
 extern "C" double cpm_stencil_df_error_bound(const cpm_stencil *S) {
@@ -1030,6 +1182,16 @@ extern "C" size_t cpm_cg_stencil_workspace_bytes(int64_t unknowns, int nrhs, int
   using namespace cpm;
   const size_t base = layout(unknowns, nrhs, precision ? 1 : 0, nullptr, nullptr);
   return precision ? base + align256(sizeof(float) * (size_t)unknowns * nrhs) : base;
+}
+
+extern "C" size_t cpm_cg_stencil_workspace(const cpm_stencil *S, int nrhs, int precision) {
+  using namespace cpm;
+  if (!S || S->nx < 3 || S->ny < 3 || S->nz < 3 || (S->ncomp != 1 && S->ncomp != 3) || (nrhs != 1 && nrhs != 3))
+    return 0;
+  const size_t cg = cpm_cg_stencil_workspace_bytes((int64_t)S->nx * S->ny * S->nz * S->ncomp, nrhs, precision);
+  if (!precision || S->ncomp != 1) return cg;
+  const size_t ch = head_bytes() + 5 * align256(sizeof(float) * cheb_vec_floats(S->nx, S->ny, S->nz, nrhs));
+  return std::max(cg, ch);
 }
 
 extern "C" int cpm_stencil_apply(const cpm_stencil *S, const double *x, double *y, double alpha, int nvec,

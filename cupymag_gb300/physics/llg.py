@@ -49,7 +49,8 @@ SOLVE_NAMES = ["elasticity", "demag", "Gauss-Seidel g1n/g2n/g3n", "Gauss-Seidel 
 # iterations); the Gauss-Seidel solves (A1, A2; ~30-55 iterations) converge in the same
 # iterations down to 1e-5, so fewer FP64 products win: at 128^3 (cold, 1 and 3 right-hand sides)
 # 1e-4 takes three FP64 residuals, 1e-5 two at the same iteration counts (7-10 % faster), 1e-6
-# adds an iteration; demag is best near 1e-3.
+# adds an iteration; demag is best near 1e-3.  On stencil operators A1 and A2 run Chebyshev cycles instead
+# (csrc/cheby.cuh), which set their own interval; the factor serves their CSR form.
 INNER_TOL = [0.1, 1e-3, 1e-5, 1e-5, 1e-5, 1e-5]
 
 # Solves that the precision form runs with the FFT solver on stencil operators: elasticity and demag,

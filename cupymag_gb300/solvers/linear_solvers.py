@@ -34,17 +34,19 @@ class CGSolver:
         self.inner_tol = 0.1   # reliable-update factor of the mixed-precision solver
         self.max_outer = 60
         self.fft_layout = N.FFT_LAYOUT_AUTO  # spectrum layout of the FFT solves
-        # FP32 stencil solves: workspace for double-float residual passes where their error bound allows
-        # (False: every reliable update takes an FP64 residual)
+        # FP32 stencil solves: double-float residual passes where their error bound allows (False: every true
+        # residual is FP64)
         self.df_residual = True
 
-    def workspace(self, n, nrhs, prec, stencil=False):
-        """Device workspace of a solve; stencil operators take the size that enables every form."""
-        key = (n, nrhs, prec, stencil)
+    def workspace(self, n, nrhs, prec, stencil=None):
+        """Device workspace of a solve; stencil operators (`stencil`: the operator) take the size that enables
+        every form."""
+        key = (n, nrhs, prec, None if stencil is None else (stencil.nx, stencil.ny, stencil.nz))
         ws = self._ws.get(key)
         if ws is None:
-            query = N.lib().cpm_cg_stencil_workspace_bytes if stencil else N.lib().cpm_cg_workspace_bytes
-            nbytes = query(n, nrhs, prec)
+            L = N.lib()
+            nbytes = L.cpm_cg_workspace_bytes(n, nrhs, prec) if stencil is None else \
+                L.cpm_cg_stencil_workspace(stencil.struct(), nrhs, prec)
             ws = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
             self._ws[key] = ws
         return ws
@@ -54,7 +56,8 @@ class CGSolver:
                precond=None, carry=None):
         """Asynchronous solve; x is read as x0 when use_init, and overwritten.
 
-        form (FP32 stencil solves): N.CG_FORM_DEFAULT (three grid barriers per iteration),
+        form (FP32 stencil solves): N.CG_FORM_DEFAULT (Chebyshev steps where the operator's symbol bounds
+        its spectrum, as for A1 and A2; CG with three grid barriers per iteration otherwise),
         N.CG_FORM_THREE_BARRIER or N.CG_FORM_TWO_BARRIER (opt-in).
         precond="fft" (FP32 form on a stencil operator with one right-hand side): FP64 refinement
         whose steps solve with the operator's circulant inverse, exactly (one FFT solve per step)
@@ -76,7 +79,7 @@ class CGSolver:
         if not (b.is_contiguous() and x.is_contiguous()) or b.dtype != torch.float64 or x.dtype != torch.float64:
             raise TypeError("b and x must be contiguous float64 device tensors")
         stencil = hasattr(A, "ncomp")
-        ws = self.workspace(n, nrhs, prec, stencil=stencil and self.df_residual)
+        ws = self.workspace(n, nrhs, prec, stencil=A if stencil else None)
         o = N.CGOpts()
         o.tol = float(tol)
         o.maxiter = int(maxiter)
@@ -86,6 +89,8 @@ class CGSolver:
         o.inner_tol = self.inner_tol if inner_tol is None else float(inner_tol)
         o.max_outer = self.max_outer
         o.form = int(form)
+        if stencil and prec == 1 and form == N.CG_FORM_DEFAULT and not self.df_residual:
+            o.form = N.CG_FORM_FP64_RESIDUALS
         o.barrier_timeout_s = self.barrier_timeout_s
         fn = N.lib().cpm_cg_solve_stencil if stencil else N.lib().cpm_cg_solve
         N.check(fn(A.struct(), b.data_ptr(), x.data_ptr(), nrhs, C.byref(o), ws.data_ptr(), ws.numel(),

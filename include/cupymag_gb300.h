@@ -65,8 +65,8 @@ typedef struct {
   int32_t precision;       /* 0 = FP64 CG, 1 = FP32 CG with reliable updates on FP64 (or proven double-float) residuals */
   double inner_tol;        /* reliable update when the FP32 residual fell by this factor (default 0.1) */
   int32_t max_outer;       /* unused (kept for layout) */
-  int32_t form;            /* FP32 stencil solvers: CPM_CG_FORM_DEFAULT (= three grid barriers per
-                              iteration), CPM_CG_FORM_THREE_BARRIER, CPM_CG_FORM_TWO_BARRIER;
+  int32_t form;            /* FP32 stencil solvers: CPM_CG_FORM_DEFAULT, CPM_CG_FORM_THREE_BARRIER,
+                              CPM_CG_FORM_TWO_BARRIER, CPM_CG_FORM_FP64_RESIDUALS;
                               FFT solves: CPM_CG_FORM_DEFAULT (direct refinement with an anchored
                               plan) or CPM_CG_FORM_FFT_PCG */
   double barrier_timeout_s;/* bound on every grid-barrier wait (seconds) */
@@ -83,13 +83,17 @@ typedef struct {
   int32_t *carry_valid;
 } cpm_cg_opts;
 
-/* Iteration forms of the FP32 stencil CG (cpm_cg_opts.form).  Both run CG to
+/* Iteration forms of the FP32 stencil CG (cpm_cg_opts.form).  DEFAULT is the
+ * Chebyshev iteration for the scalar stencils whose symbol bounds it (see
+ * cpm_cg_stencil_workspace) and three grid barriers per CG iteration otherwise;
+ * FP64_RESIDUALS is DEFAULT with every true residual in FP64.  The two CG forms run CG to
  * the same FP64 stopping test; the two-barrier form keeps s ~ A p beside p and
  * forms A r in its one product, so an iteration needs one reduction of four
  * sums instead of two reductions and a third barrier.  The two-barrier form is
  * opt-in: on GB300 it measured slower per iteration, and its FP32 recurrences
  * drift enough to stall the 128^3 elastic and demag solves. */
-enum { CPM_CG_FORM_DEFAULT = 0, CPM_CG_FORM_THREE_BARRIER = 1, CPM_CG_FORM_TWO_BARRIER = 2, CPM_CG_FORM_FFT_PCG = 3 };
+enum { CPM_CG_FORM_DEFAULT = 0, CPM_CG_FORM_THREE_BARRIER = 1, CPM_CG_FORM_TWO_BARRIER = 2, CPM_CG_FORM_FFT_PCG = 3,
+       CPM_CG_FORM_FP64_RESIDUALS = 4 };
 
 /* ---- library ---- */
 const char *cpm_version(void);
@@ -195,6 +199,14 @@ int cpm_stencil_apply32(const cpm_stencil *S, const float *x, float *y, int nvec
 int cpm_cg_solve_stencil(const cpm_stencil *S, const double *b, double *x, int nrhs, const cpm_cg_opts *opts,
                          void *workspace, size_t workspace_bytes, cpm_cg_info *info_dev, void *stream);
 size_t cpm_cg_stencil_workspace_bytes(int64_t unknowns, int nrhs, int precision);
+/* Workspace bytes for every form of a solve on this operator (only the grid and ncomp are read).  With that
+ * much, the FP32 form of a scalar stencil that is even along every axis, with a positive symbol of condition
+ * number at most 64, runs Chebyshev steps between its true residuals in place of CG: on the free DOFs the
+ * operator's spectrum lies between the symbol's extremes, so the steps need no inner products (one grid
+ * barrier and 16 bytes per unknown each).  Same stopping test and statuses; info->iters counts the steps
+ * (40 and 61 where CG takes 28-36 and 41-55 on A1 and A2).  maxiter below four times a cold start's
+ * steps, and flagged rows that are not pinned, keep CG. */
+size_t cpm_cg_stencil_workspace(const cpm_stencil *S, int nrhs, int precision);
 /* The bound behind that choice, as a multiple of ||b||: 2 g sum|c| / sigma_min with g = 128 * 2^-48 and
  * sigma_min a lower bound of the stencil's symbol (its part even along every axis is minimised over the 8
  * corners cos theta = +-1, the rest bounded by the sum of its magnitudes); -1 where sigma_min <= 0 or the
