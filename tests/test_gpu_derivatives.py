@@ -1,0 +1,55 @@
+"""The marching derivative kernels (csrc/deriv.cu, mirror_kernel) against the pair kernels."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _nearly(c):
+    """The stencils with 1e-13 of their largest coefficient moved (c(d) up, c(-d) down): odd to 1e-12, so the pair
+    kernels take them, but not mirror symmetric to 1e-15, so the marching kernels do not."""
+    c = np.array(c, dtype=np.float64).reshape(-1, 27)
+    e = 1e-13 * np.abs(c).max()
+    c[:, 3] += e
+    c[:, 23] -= e
+    return c, e
+
+
+# tiles that end inside the grid, one-row and one-column remainders, planes split unevenly, the shortest axes
+@pytest.mark.parametrize("dims", [(33, 50, 61), (3, 200, 140), (150, 3, 190), (200, 140, 3), (47, 46, 45),
+                                  (64, 40, 33)])
+def test_marching_products_match_the_pair_kernels(dims):
+    """A moved coefficient changes each output by at most 2 e max|x| per stencil it enters (e = 1e-13 of the largest
+    coefficient); rounding adds less than 1e-14 of the largest output."""
+    from cupymag_gb300.core.assemble_simulation_operators import SimulationOperators
+    from cupymag_gb300.utils.stencil_derivatives import StencilCoupling, StencilDerivatives
+    from cupymag_gb300.workloads import hex_params
+    cell = SimulationOperators(hex_params(6, 1, True, True), device="cuda")
+    fx, fy, fz = cell.stencil_derivatives().coef
+    fel = cell.stencil_coupling().coef
+    n = dims[0] * dims[1] * dims[2]
+    (gx, ex), (gy, ey), (gz, ez) = (_nearly(f) for f in (fx, fy, fz))
+    gel, eel = _nearly(fel)
+    D, D2 = StencilDerivatives(*dims, fx, fy, fz), StencilDerivatives(*dims, gx, gy, gz)
+    F, F2 = StencilCoupling(*dims, fel), StencilCoupling(*dims, gel.reshape(-1))
+    rng = np.random.default_rng(sum(dims))
+    dev = lambda *s: torch.as_tensor(rng.normal(size=s), device="cuda")  # noqa: E731
+    new = lambda *s: torch.empty(s, dtype=torch.float64, device="cuda")  # noqa: E731
+
+    def close(a, b, bound, what):
+        assert float((a - b).abs().max()) <= bound + 1e-14 * float(b.abs().max()), what
+
+    U, m, avg, u, E0 = dev(n), dev(n, 3), dev(3), dev(3 * n), dev(6 * n)
+    big = lambda x: float(x.abs().max())  # noqa: E731
+    close(D.hd_into(U, new(n, 3)), D2.hd_into(U, new(n, 3)), 2 * max(ex, ey, ez) * big(U), "Hd")
+    a, b = D.demag_rhs_into(m, avg, new(n), pin=5), D2.demag_rhs_into(m, avg, new(n), pin=5)
+    close(a, b, 2 * (ex + ey + ez) * big(m), "right-hand side")
+    assert float(a[5]) == 0.0
+    R = torch.as_tensor(np.linalg.qr(rng.normal(size=(3, 3)))[0], device="cuda")
+    for rot in (None, R):
+        # at most 6 derivatives enter a rotated component, each times at most 1
+        close(D.compute_E_from_u(n, u, rot), D2.compute_E_from_u(n, u, rot), 12 * max(ex, ey, ez) * big(u), "strain")
+    a, b = F.spmv(E0), F2.spmv(E0)
+    close(a, b, 12 * eel * big(E0), "F_el E0")
+    assert float(a[0]) == float(a[n]) == float(a[2 * n]) == 0.0
