@@ -61,7 +61,8 @@ class BatchSystem(C.Structure):
 
 class BatchPlan(C.Structure):
     _fields_ = [("dev", vp), ("bytes", i64), ("nsys", i32), ("grid", i32), ("ncomp", i32), ("nrhs", i32),
-                ("precision", i32), ("total_chunks", i32), ("coef", dbl * 243)]
+                ("precision", i32), ("total_chunks", i32), ("coef", dbl * 243), ("cheb", i64), ("cheb_nsys", i32),
+                ("cheb_grid", i32)]
 
 
 class DerivStencilC(C.Structure):

@@ -31,6 +31,7 @@
 #include <cmath>
 #include <vector>
 
+#include "cheby.cuh"
 #include "stencil_ops.cuh"
 
 namespace cpm {
@@ -69,6 +70,8 @@ struct BatchArgs {
   long long half;
   GridBarrier *bar;
   int *live;             // systems (segments) still iterating
+  const int *done;       // per segment: solved by the Chebyshev launch (NULL: none); done[nsys]: how many
+  int nsys;
   unsigned long long timeout_ns;
   double inner_tol;
 };
@@ -357,6 +360,7 @@ __global__ void __launch_bounds__(kCGThreads, (NC == 1 && NR == 3) ? 3 : 4) cg_b
     const __grid_constant__ BatchArgs a) {
   constexpr int U = NC * NR;
   constexpr int NS = b_systems<NC, NR>();
+  if (a.done && __ldcg(a.done + a.nsys) == a.nsys) return;  // (all CTAs)
   __shared__ double s_red[9][kCGWarps];
   __shared__ double s_stage[kStageDoubles];
   __shared__ IRState st[NS];
@@ -377,10 +381,13 @@ __global__ void __launch_bounds__(kCGThreads, (NC == 1 && NR == 3) ? 3 : 4) cg_b
   const bool use_init = S.use_init_dev && __ldcg(S.use_init_dev) != 0;
   const bool quads = S.quads != 0;  // chunks are multiples of 4 DOFs
   int par = 0;
+  const bool skip = a.done && __ldcg(a.done + a.cta_seg[blockIdx.x]) != 0;
 
   // ---- r = b - A64 x, r32 = p32 = r, d = 0; ||b||, ||r||
   double v[2 * NS];
-  bool ok = seg_reduce<2 * NS>(a, S, l, true, par, s_red, s_stage, v, [&](int d0, int d1, double (&w)[2 * NS]) {
+#pragma unroll
+  for (int j = 0; j < 2 * NS; ++j) v[j] = 0.0;
+  bool ok = seg_reduce<2 * NS>(a, S, l, !skip, par, s_red, s_stage, v, [&](int d0, int d1, double (&w)[2 * NS]) {
     for (int dof = d0 + threadIdx.x; dof < d1; dof += kCGThreads) {
       double y[U];
       if (use_init) apply_c<double, NC, NR>(g, a.c64, x, dof, y);
@@ -405,9 +412,9 @@ __global__ void __launch_bounds__(kCGThreads, (NC == 1 && NR == 3) ? 3 : 4) cg_b
       const double bn = ok ? sqrt(v[j]) : 0.0;
       ir_init(st[j], bn, ok ? v[NS + j] : 0.0, S.tol);
       am |= st[j].active << j;
-      if (lead) S.info->bnorm[j] = bn;
+      if (lead && !skip) S.info->bnorm[j] = bn;
     }
-    if (lead) {
+    if (lead && !skip) {
       for (int j = NS; j < 3; ++j) S.info->bnorm[j] = 0.0;
       if (am) atomicAdd(a.live, 1);
     }
@@ -418,7 +425,7 @@ __global__ void __launch_bounds__(kCGThreads, (NC == 1 && NR == 3) ? 3 : 4) cg_b
   __syncthreads();
   int activem = s_mask[0], needm = 0;
   int status = ok ? CPM_OK : CPM_BARRIER_TIMEOUT;
-  if (ok && use_init) {
+  if (ok && use_init && !skip) {
     for (int cc = l; cc < S.nchunks; cc += S.ncta) {
       const int d1 = min(g.n, (cc + 1) * S.chunk_dofs);
       for (int dof = cc * S.chunk_dofs + threadIdx.x; dof < d1; dof += kCGThreads)
@@ -592,7 +599,7 @@ __global__ void __launch_bounds__(kCGThreads, (NC == 1 && NR == 3) ? 3 : 4) cg_b
       }
     }
   }
-  if (lead && threadIdx.x == 0) {
+  if (lead && threadIdx.x == 0 && !skip) {
     int sta = status;
     if (*(volatile const int *)&a.bar->error && sta == CPM_OK) sta = CPM_BARRIER_TIMEOUT;
     for (int j = 0; j < 3; ++j) {
@@ -880,6 +887,35 @@ __global__ void __launch_bounds__(kCGThreads, (NC == 1 && NR == 3) ? 3 : 4) cg_b
   }
 }
 
+// ---------------------------------------------------------------- Chebyshev iteration (csrc/cheby.cuh)
+// Every system on CTAs and a barrier of its own, with the step passes cut for those CTAs; the systems that it does not
+// fit (see cheb_solve) are left to the CG launch that follows.
+struct ChebBatchArgs {
+  ChebOp op;
+  const ChebSys *sys;
+  const int *cta_sys, *seg;  // CTA -> system, system -> segment of the plan
+  int *done;
+  int nsys;                  // segments of the plan
+};
+
+template <int NR>
+__global__ void __launch_bounds__(kChebThreads, kChebBlocks) cheb_batched_kernel(
+    const __grid_constant__ ChebBatchArgs a) {
+  __shared__ double s_red[NR + 1][kCGWarps];
+  __shared__ ChebSys s_sys;
+  const int id = a.cta_sys[blockIdx.x];
+  if (threadIdx.x == 0) {
+    s_sys = a.sys[id];
+    if (blockIdx.x == s_sys.cta0) s_sys.info->status = CPM_OK;
+  }
+  __syncthreads();
+  const int l = blockIdx.x - s_sys.cta0;
+  if (cheb_solve<NR>(s_sys, a.op, l, s_red) && l == 0 && threadIdx.x == 0) {
+    a.done[a.seg[id]] = 1;
+    atomicAdd(a.done + a.nsys, 1);
+  }
+}
+
 // ---------------------------------------------------------------- host side
 // DOFs per chunk of one system: a base size per operator kind, doubled until
 // the system has at most kMaxChunks chunks.  It depends on the system alone,
@@ -924,6 +960,47 @@ static PlanLayout plan_layout(int64_t total_chunks, int nsys, int grid) {
   L.ctamap = L.segs + align256(sizeof(BSeg) * (size_t)nsys);
   L.total = L.ctamap + align256(sizeof(int) * (size_t)grid);
   return L;
+}
+
+// The Chebyshev part of a plan, from `at` in plan memory: control words (barriers, done flags), the system table,
+// the CTA and segment maps, partials, vectors.
+struct ChebLayout {
+  size_t bars, done, ctl, sys, ctamap, seg, part, total;
+};
+
+static ChebLayout cheb_plan_layout(size_t at, int nsys, int grid) {
+  ChebLayout L;
+  L.bars = at;
+  L.done = L.bars + align256(sizeof(GridBarrier) * (size_t)nsys);
+  L.ctl = L.done + align256(sizeof(int) * (size_t)(nsys + 1)) - at;
+  L.sys = at + L.ctl;
+  L.ctamap = L.sys + align256(sizeof(ChebSys) * (size_t)nsys);
+  L.seg = L.ctamap + align256(sizeof(int) * (size_t)grid);
+  L.part = L.seg + align256(sizeof(int) * (size_t)nsys);
+  L.total = L.part;
+  return L;
+}
+
+// Bytes of the vectors and partials of one system.
+static size_t cheb_sys_bytes(const cpm_batch_system &y, int nrhs, int sms) {
+  ChebSys S{};
+  S.nx = y.nx;
+  S.ny = y.ny;
+  S.nz = y.nz;
+  S.n = y.nx * y.ny * y.nz;
+  cheb_layout(S, nrhs, sms);
+  return align256(sizeof(double) * 2 * (size_t)S.half) +
+         5 * align256(sizeof(float) * cheb_vec_floats(y.nx, y.ny, y.nz, nrhs));
+}
+
+static int cheb_max_grid() { return sm_count() * kChebBlocks; }
+
+// Bytes of the Chebyshev part (0 where the plan has none).
+static size_t cheb_part_bytes(const cpm_batch_system *sys, int nsys, int ncomp, int nrhs, int precision) {
+  if (ncomp != 1 || !precision || nsys > cheb_max_grid()) return 0;
+  size_t b = cheb_plan_layout(0, nsys, cheb_max_grid()).total;
+  for (int s = 0; s < nsys; ++s) b += cheb_sys_bytes(sys[s], nrhs, sm_count());
+  return b;
 }
 
 struct Assignment {
@@ -1012,7 +1089,8 @@ extern "C" int cpm_batch_plan_bytes(const cpm_batch_system *sys, int32_t nsys, i
     set_error("cpm_batch_plan_bytes: bytes is NULL");
     return CPM_BAD_ARG;
   }
-  *bytes = (int64_t)plan_layout(A.total_chunks, nsys, A.grid).total;
+  *bytes = (int64_t)(plan_layout(A.total_chunks, nsys, A.grid).total +
+                     cheb_part_bytes(sys, nsys, ncomp, nrhs, precision));
   return CPM_OK;
 }
 
@@ -1023,9 +1101,10 @@ extern "C" int cpm_batch_plan_build(const cpm_batch_system *sys, int32_t nsys, i
   Assignment A;
   if (int e = assign(sys, nsys, ncomp, nrhs, precision, A, "cpm_batch_plan_build")) return e;
   const PlanLayout L = plan_layout(A.total_chunks, nsys, A.grid);
-  if (!coef || !plan || !plan_dev || plan_bytes < (int64_t)L.total || ((uintptr_t)plan_dev & 255)) {
+  const size_t total = L.total + cheb_part_bytes(sys, nsys, ncomp, nrhs, precision);
+  if (!coef || !plan || !plan_dev || plan_bytes < (int64_t)total || ((uintptr_t)plan_dev & 255)) {
     set_error("cpm_batch_plan_build: bad arguments (coef, plan and a 256-byte aligned device buffer of at least "
-              "%zu bytes)", L.total);
+              "%zu bytes)", total);
     return CPM_BAD_ARG;
   }
   std::vector<BSeg> segs(nsys);
@@ -1073,11 +1152,82 @@ extern "C" int cpm_batch_plan_build(const cpm_batch_system *sys, int32_t nsys, i
   }
   cudaStream_t st = (cudaStream_t)stream;
   char *base = (char *)plan_dev;
+  plan->cheb = 0;
+  plan->cheb_nsys = plan->cheb_grid = 0;
+  std::vector<ChebSys> csys;
+  std::vector<int> cseg, ccta;
+  ChebLayout CL{};
+  if (total > L.total) {
+    // the systems that the single solver would run with Chebyshev steps, by the same rule
+    cpm_stencil one{};
+    one.ncomp = 1;
+    for (int i = 0; i < 27; ++i) one.coef[i] = coef[i];
+    ChebOp op;
+    const double e = df_error_bound(&one);
+    if (e > 0.0 && cheb_operator(coef, 1, &op)) {
+      const int sms = sm_count(), gmax = cheb_max_grid();
+      int64_t work = 0;
+      CL = cheb_plan_layout(L.total, nsys, gmax);
+      size_t at = CL.total;
+      for (int s = 0; s < nsys; ++s) {
+        const cpm_batch_system &y = sys[s];
+        if (!(e <= 0.25 * y.tol) || y.maxiter < 4 * cheb_cold_steps(op, y.tol)) continue;
+        ChebSys S{};
+        S.nx = y.nx;
+        S.ny = y.ny;
+        S.nz = y.nz;
+        S.n = y.nx * y.ny * y.nz;
+        S.flags = y.flags;
+        S.b = y.b;
+        S.x = y.x;
+        S.use_init_dev = y.use_init_dev;
+        S.maxiter = y.maxiter;
+        S.tol = y.tol;
+        S.info = y.info;
+        cheb_layout(S, nrhs, sms);
+        S.part = (double *)(base + at);
+        at += align256(sizeof(double) * 2 * (size_t)S.half);
+        for (int k = 0; k < 5; ++k) {
+          S.v[k] = (float *)(base + at) + kChebPad;
+          at += align256(sizeof(float) * cheb_vec_floats(y.nx, y.ny, y.nz, nrhs));
+        }
+        S.bar = (GridBarrier *)(base + CL.bars) + csys.size();
+        work += S.n;
+        cseg.push_back(s);
+        csys.push_back(S);
+      }
+      // CTAs by size; a system's step passes are cut for its CTAs (its sums keep the cut of the system alone)
+      for (size_t s = 0; s < csys.size(); ++s) {
+        ChebSys &S = csys[s];
+        const int64_t spare = gmax - (int64_t)csys.size();
+        const int share = 1 + (int)(spare * S.n / work);
+        const int tiles = S.chunks / S.ranges;
+        cheb_split(S.nx, tiles, std::max(1, share / kChebBlocks), share, S.lx, S.ranges);
+        S.chunks = tiles * S.ranges;
+        S.cta0 = (int)ccta.size();
+        S.ncta = std::min(share, S.chunks);
+        ccta.insert(ccta.end(), S.ncta, (int)s);
+      }
+    }
+  }
+  if (!csys.empty()) {
+    int occ = 0;
+    const void *fn = nrhs == 3 ? (const void *)cheb_batched_kernel<3> : (const void *)cheb_batched_kernel<1>;
+    CPM_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kChebThreads, 0));
+    if ((int64_t)occ * sm_count() >= (int64_t)ccta.size()) {
+      plan->cheb = (int64_t)L.total;
+      plan->cheb_nsys = (int32_t)csys.size();
+      plan->cheb_grid = (int32_t)ccta.size();
+      CPM_TRY(cudaMemcpyAsync(base + CL.sys, csys.data(), sizeof(ChebSys) * csys.size(), cudaMemcpyHostToDevice, st));
+      CPM_TRY(cudaMemcpyAsync(base + CL.seg, cseg.data(), sizeof(int) * cseg.size(), cudaMemcpyHostToDevice, st));
+      CPM_TRY(cudaMemcpyAsync(base + CL.ctamap, ccta.data(), sizeof(int) * ccta.size(), cudaMemcpyHostToDevice, st));
+    }
+  }
   CPM_TRY(cudaMemcpyAsync(base + L.segs, segs.data(), sizeof(BSeg) * nsys, cudaMemcpyHostToDevice, st));
   CPM_TRY(cudaMemcpyAsync(base + L.ctamap, cmap.data(), sizeof(int) * A.grid, cudaMemcpyHostToDevice, st));
   CPM_TRY(cudaStreamSynchronize(st));  // the staging vectors go out of scope
   plan->dev = plan_dev;
-  plan->bytes = (int64_t)L.total;
+  plan->bytes = (int64_t)total;
   plan->nsys = nsys;
   plan->grid = A.grid;
   plan->ncomp = ncomp;
@@ -1112,6 +1262,29 @@ extern "C" int cpm_cg_solve_blockdiag(const cpm_batch_plan *plan, const cpm_cg_o
   a.timeout_ns = (unsigned long long)(tmo * 1e9);
   a.inner_tol = opts->inner_tol > 0 ? opts->inner_tol : 0.1;
   cudaStream_t st = (cudaStream_t)stream;
+  if (plan->cheb_grid > 0 &&
+      (opts->form == CPM_CG_FORM_DEFAULT || opts->form == CPM_CG_FORM_FP64_RESIDUALS)) {
+    const ChebLayout CL = cheb_plan_layout((size_t)plan->cheb, plan->nsys, cheb_max_grid());
+    ChebBatchArgs c;
+    cpm_stencil one{};
+    one.ncomp = 1;
+    for (int i = 0; i < 27; ++i) one.coef[i] = plan->coef[i];
+    cheb_operator(plan->coef, 1, &c.op);
+    c.op.df = opts->form == CPM_CG_FORM_DEFAULT;
+    c.op.df_err = df_error_bound(&one);
+    c.op.timeout_ns = a.timeout_ns;
+    c.sys = (const ChebSys *)(base + CL.sys);
+    c.cta_sys = (const int *)(base + CL.ctamap);
+    c.seg = (const int *)(base + CL.seg);
+    c.done = (int *)(base + CL.done);
+    c.nsys = plan->nsys;
+    a.done = c.done;
+    a.nsys = plan->nsys;
+    CPM_TRY(cudaMemsetAsync(base + plan->cheb, 0, CL.ctl, st));
+    void *cargs[] = {&c};
+    const void *fn = plan->nrhs == 3 ? (const void *)cheb_batched_kernel<3> : (const void *)cheb_batched_kernel<1>;
+    CPM_TRY(cudaLaunchCooperativeKernel(fn, dim3(plan->cheb_grid), dim3(kChebThreads), cargs, 0, st));
+  }
   CPM_TRY(cudaMemsetAsync(base + L.bar, 0, 32, st));
   void *args[] = {&a};
   CPM_TRY(cudaLaunchCooperativeKernel(batched_kernel(plan->ncomp, plan->nrhs, plan->precision, opts->form),

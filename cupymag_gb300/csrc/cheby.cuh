@@ -37,8 +37,8 @@
 // unevaluated sum h + l of two float vectors until the end.  A right-hand side
 // whose norm leaves the middle of the float range is solved as 2^-e b.
 //
-// A system's chunks (runs of a plane times a range of planes) and all its sums
-// depend on the system alone, and its CTAs pass a grid barrier of their own.
+// The chunks of the passes that sum (runs of a plane times a range of planes) depend on the system alone, and its
+// CTAs pass a grid barrier of their own: a system's iterates are the same bits on any number of CTAs.
 #pragma once
 
 #include "stencil_ops.cuh"
@@ -81,6 +81,7 @@ struct ChebSys {
   GridBarrier *bar;
   int pitch, nq;                      // floats and quads of a z-line
   int runs, tw, lx, ranges, chunks;   // step passes: runs of 32 quads per plane, runs per tile, planes per range
+  int clx, cranges, cchunks;          // the check's passes, on the same tiles
   int rtiles, rlx, rranges, rchunks;  // residual passes: tiles of kChebThreads DOFs of a plane
   int lchunk, lchunks;                // pointwise passes: z-lines per chunk
   int cta0, ncta;
@@ -126,6 +127,9 @@ inline void cheb_layout(ChebSys &S, int nrhs, int sms) {
   tiles = (S.runs + S.tw - 1) / S.tw;
   cheb_split(S.nx, tiles, sms, slots, S.lx, S.ranges);
   S.chunks = tiles * S.ranges;
+  S.clx = S.lx;
+  S.cranges = S.ranges;
+  S.cchunks = S.chunks;
   S.rtiles = (int)(((int64_t)S.ny * S.nz + kChebThreads - 1) / kChebThreads);
   cheb_split(S.nx, S.rtiles, sms, slots, S.rlx, S.rranges);
   S.rchunks = S.rtiles * S.rranges;
@@ -133,13 +137,15 @@ inline void cheb_layout(ChebSys &S, int nrhs, int sms) {
   S.lchunk = lc < per ? per : lc;
   S.lchunks = (lines + S.lchunk - 1) / S.lchunk;
   const int most = S.rchunks > S.lchunks ? S.rchunks : S.lchunks;
-  S.half = kChebSlot * (S.chunks > most ? S.chunks : most);
+  S.half = kChebSlot * (S.cchunks > most ? S.cchunks : most);
 }
 
 // Whether the iteration applies to a stencil at all, and its factors: scalar, even along every axis to
 // rounding, symbol positive with a condition number of at most 64 (CG's iterations grow more slowly on
 // wider spectra).
 bool cheb_operator(const double *coef, int ncomp, ChebOp *op);
+// Error bound of a double-float residual as a multiple of ||b|| (-1: none).
+double df_error_bound(const cpm_stencil *s);
 // Steps that the iteration takes from a cold start to tol (host estimate of the device's schedule).
 int cheb_cold_steps(const ChebOp &op, double tol);
 
@@ -297,8 +303,9 @@ __device__ __forceinline__ void cheb_pass(const ChebSys &S, const ChebOp &op, in
     co[e] = pack2(t, t);
   }
   const f32x2 cb2 = pack2(cb, cb), cg2 = pack2(cg, cg);
-  for (int chunk = l; chunk < S.chunks; chunk += S.ncta) {
-    const int tile = chunk / S.ranges, x0 = (chunk - tile * S.ranges) * S.lx, x1 = min(nx, x0 + S.lx);
+  const int lx = CHECK ? S.clx : S.lx, ranges = CHECK ? S.cranges : S.ranges, chunks = CHECK ? S.cchunks : S.chunks;
+  for (int chunk = l; chunk < chunks; chunk += S.ncta) {
+    const int tile = chunk / ranges, x0 = (chunk - tile * ranges) * lx, x1 = min(nx, x0 + lx);
     const int run = tile * S.tw + warp;
     float sum = 0.0f;
     int rhs = 0;
@@ -732,7 +739,7 @@ __device__ __forceinline__ bool cheb_solve(const ChebSys &S, const ChebOp &op, i
         double *half = S.part + (size_t)par * S.half;
         cheb_pass<NR, true>(S, op, l, d0, d1, r, 0.0f, 0.0f, 1.0f, 1.0f, scale, half, sred);
         double t[NR];
-        if (!cheb_totals<NR>(S, tns, S.chunks, par, t, sred)) { status = CPM_BARRIER_TIMEOUT; break; }
+        if (!cheb_totals<NR>(S, tns, S.cchunks, par, t, sred)) { status = CPM_BARRIER_TIMEOUT; break; }
         if (threadIdx.x == 0) {
           int left = 0;
           for (int s = 0; s < NR; ++s) {

@@ -894,7 +894,7 @@ static int check_stencil(const cpm_stencil *s, const char *who) {
 // minimum is at one of the 8 corners cos = +-1; the rest of c moves sigma by at most the sum of its
 // magnitudes.  With e = g sum|c| / sigma_min, a residual with ||t_df|| <= tol ||b|| - 2 e ||b|| has
 // ||t|| <= (tol ||b|| - e ||b||) / (1 - e) <= tol ||b||: the bound returned is 2 e.
-static double df_error_bound(const cpm_stencil *s) {
+double df_error_bound(const cpm_stencil *s) {
   if (s->ncomp != 1) return -1.0;
   const double *c = s->coef;
   double even[27], s1 = 0.0, odd = 0.0;

@@ -65,7 +65,13 @@ def estimate_bytes(p, precision="IR") -> int:
         # FFT solves: workspace (five FP32 vectors and a complex field of 3n unknowns) and the plans'
         # inverse symbols (6 floats per DOF elastic, 1 demag)
         per += 3 * (20 + 8) + 4 * (6 + 1)
-    return int(per * n * 1.05) + (8 << 20)
+    cheb = 0
+    if precision != "DP":
+        # Chebyshev solves: five FP32 vectors of padded z-lines per right-hand side of the projection plans (3, 1, 1
+        # and 3) and, in small runs, of the demag plan
+        pitch = (int(p.Nz) + 9) // 8 * 8
+        cheb = 5 * 4 * int(p.Nx) * int(p.Ny) * pitch * (8 if n >= FFT_MIN_DOFS else 9)
+    return int((per * n + cheb) * 1.05) + (8 << 20)
 
 
 @dataclass

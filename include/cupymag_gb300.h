@@ -240,6 +240,8 @@ typedef struct {
   int64_t bytes;
   int32_t nsys, grid, ncomp, nrhs, precision, total_chunks;
   double coef[243];
+  int64_t cheb;            /* offset of the Chebyshev part in dev (scalar operators, precision 1), or 0 */
+  int32_t cheb_nsys, cheb_grid; /* its systems and CTAs (0: every system runs CG) */
 } cpm_batch_plan;
 
 /* Work-vector bytes of one system on an nx x ny x nz grid; 0 for invalid dimensions. */
@@ -258,7 +260,9 @@ int cpm_batch_plan_build(const cpm_batch_system *sys, int32_t nsys, int32_t ncom
                          cpm_batch_plan *plan, void *stream);
 
 /* Solve every system of the plan in one cooperative launch on `stream`
- * (a memset and a kernel: the call can be captured in a CUDA graph).  opts:
+ * (a memset and a kernel: the call can be captured in a CUDA graph).  In precision 1 scalar systems that
+ * cpm_cg_solve_stencil would run with Chebyshev steps do so here too, each on CTAs and a grid barrier of its
+ * own (a launch before the CG one, which then serves the systems left and ends at once when there are none).  opts:
  * inner_tol and barrier_timeout_s are used; tolerances, maxiter and
  * warm-start flags come from the systems. */
 int cpm_cg_solve_blockdiag(const cpm_batch_plan *plan, const cpm_cg_opts *opts, void *stream);

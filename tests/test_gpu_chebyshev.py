@@ -102,3 +102,54 @@ def test_rows_that_are_not_pinned_and_small_maxiter_keep_cg():
         _, inf = _solve(op, b, maxiter=cap)
         _, ref = _solve(op, b, maxiter=cap, form=N.CG_FORM_THREE_BARRIER)
         assert inf["iters"] == ref["iters"] and inf["status"] == ref["status"]
+
+
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_batched_chebyshev_is_the_same_alone_and_in_a_mix(nrhs):
+    """Systems of one batch that run Chebyshev steps (different grids, one with a zero right-hand side) beside ones
+    left to CG (a row that is not pinned; a maxiter below the rule): bit for bit the same alone and in the mix, the
+    stopping test holds, and the Chebyshev systems give the single solver's steps."""
+    from cupymag_gb300.serving.blockdiag import BlockDiagPlan, BlockSystem, work_bytes
+    from cupymag_gb300.solvers.linear_solvers import decode_info, new_info
+    from cupymag_gb300.utils.stencil_operator import COL_EXCLUDED, ROW_IDENTITY, StencilOperator
+    rng = np.random.default_rng(nrhs)
+    coef = _case((6, 6, 6), 0)[1]["A1"].coef_host
+    ops = []
+    for dims in ((7, 9, 11), (16, 16, 16), (5, 30, 33), (24, 20, 22), (8, 8, 8), (9, 9, 9)):
+        f = np.zeros(dims[0] * dims[1] * dims[2], dtype=np.uint8)
+        f[rng.integers(0, f.size, 5)] = ROW_IDENTITY | COL_EXCLUDED
+        if dims == (8, 8, 8):
+            f[100] = ROW_IDENTITY     # its column stays: CG
+        ops.append(StencilOperator(*dims, coef, f))
+    caps = [20000, 20000, 20000, 20000, 20000, 100]
+    bs = [rng.normal(size=(o.n, nrhs)) if nrhs == 3 else rng.normal(size=o.n) for o in ops]
+    bs[4].reshape(ops[4].n, -1)[100] = 0.0
+    bs[3].reshape(ops[3].n, -1)[:, 0] = 0.0
+
+    def solve(which):
+        systems = []
+        for i in which:
+            b = torch.as_tensor(bs[i], device="cuda").contiguous()
+            work = torch.empty(work_bytes((ops[i].nx, ops[i].ny, ops[i].nz), 1, nrhs, "IR"), dtype=torch.uint8,
+                               device="cuda")
+            systems.append(BlockSystem(ops[i], b, torch.zeros_like(b), new_info(1)[0], work, TOL, caps[i]))
+        plan = BlockDiagPlan(systems, "IR", inner_tol=1e-5)
+        plan.launch()
+        first = [s.x.clone() for s in systems]
+        plan.launch()   # a plan is launched many times
+        out = [(s.x.cpu().numpy(), decode_info(s.info.cpu().numpy())) for s in systems]
+        assert all(torch.equal(a, s.x) for a, s in zip(first, systems))
+        return out
+
+    mix = solve(range(len(ops)))
+    for i, op in enumerate(ops):
+        (x, inf), = solve([i])
+        assert np.array_equal(x, mix[i][0]) and inf == mix[i][1], i
+        assert inf["status"] == 0, (i, inf)
+        b2, x2 = bs[i].reshape(op.n, -1), x.reshape(op.n, -1)
+        for r in range(b2.shape[1]):
+            y = op.spmv(torch.as_tensor(np.ascontiguousarray(x2[:, r]), device="cuda")).cpu().numpy()
+            assert np.linalg.norm(b2[:, r] - y) <= 1.001 * TOL * np.linalg.norm(b2[:, r]), (i, r)
+        if i < 4:
+            _, ref = _solve(op, bs[i])
+            assert ref["iters"] == inf["iters"] and inf["df_updates"] == ref["df_updates"], (i, inf, ref)
