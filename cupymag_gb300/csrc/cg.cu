@@ -80,6 +80,7 @@ __device__ __forceinline__ void row_range(const IT *rp, int64_t row, int64_t &s,
 template <int NR, typename IT>
 __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
   __shared__ double s_red[2 * NR][kCGWarps];
+  __shared__ CG64State<NR> st;
   extern __shared__ __align__(16) unsigned char s_tile[];
   const TileSmem tile = tile_smem(s_tile);
   const int G = a.group;
@@ -129,23 +130,21 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
     set_status(a.info, CPM_BARRIER_TIMEOUT);
     return;
   }
-  double atol[NR], rho[NR], resid[NR];
-  int active[NR], iters[NR];
-  bool any = false;
+  double bb[NR], rr0[NR];
 #pragma unroll
   for (int j = 0; j < NR; ++j) {
-    const double bn = sqrt(v[j]);
-    atol[j] = a.tol * bn;
-    rho[j] = v[NR + j];
-    resid[j] = sqrt(v[NR + j]);
-    active[j] = bn != 0.0;
-    iters[j] = 0;
-    any |= active[j] != 0;
-    if (bn == 0.0 && use_init) {
+    bb[j] = v[j];
+    rr0[j] = v[NR + j];
+  }
+  cg64_init<NR>(st, bb, rr0, a.tol, blockIdx.x == 0 ? a.info->bnorm : nullptr);
+  bool any = st.any != 0;
+  if (use_init) {
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
       // cupyx returns b itself when ||b|| == 0
-      for (int64_t row = r0 + threadIdx.x; row < r1; row += kCGThreads) a.x[row * NR + j] = a.b[row * NR + j];
+      if (!st.active[j])
+        for (int64_t row = r0 + threadIdx.x; row < r1; row += kCGThreads) a.x[row * NR + j] = a.b[row * NR + j];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.info->bnorm[j] = bn;
   }
 
   int status = CPM_OK;
@@ -166,14 +165,15 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
       }
     }
     if (!grid_sum<NR>(pq, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    cg64_alpha<NR>(st, pq);
+    if (st.bad) { status = CPM_NONFINITE; break; }
     double alpha[NR];
-    bool bad = false;
+    int active[NR];
 #pragma unroll
     for (int j = 0; j < NR; ++j) {
-      alpha[j] = active[j] ? rho[j] / pq[j] : 0.0;
-      if (active[j] && !isfinite(alpha[j])) bad = true;
+      alpha[j] = st.coef[j];
+      active[j] = st.active[j];
     }
-    if (bad) { status = CPM_NONFINITE; break; }
 
     // ---- phase 2: x += alpha p, r -= alpha q, partial r.r
     double rr[NR];
@@ -191,22 +191,16 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
       }
     }
     if (!grid_sum<NR>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
-    any = false;
+    cg64_beta<NR>(st, rr, a.maxiter);
+    if (st.bad) { status = CPM_NONFINITE; break; }
+    any = st.any != 0;
+    if (!any) break;
     double beta[NR];
 #pragma unroll
     for (int j = 0; j < NR; ++j) {
-      beta[j] = 0.0;
-      if (!active[j]) continue;
-      if (!isfinite(rr[j])) bad = true;
-      iters[j] += 1;
-      beta[j] = rr[j] / rho[j];
-      rho[j] = rr[j];
-      resid[j] = sqrt(rr[j]);
-      if (resid[j] <= atol[j]) active[j] = 0;
-      any |= active[j] != 0;
+      beta[j] = st.coef[j];
+      active[j] = st.active[j];
     }
-    if (bad) { status = CPM_NONFINITE; break; }
-    if (!any || k + 1 >= a.maxiter) break;
 
     // ---- phase 3: p = r + beta p (own rows)
     for (int64_t row = r0 + threadIdx.x; row < r1; row += kCGThreads) {
@@ -220,15 +214,14 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
     if (!grid_sync(a.bar, gridDim.x, tns)) { status = CPM_BARRIER_TIMEOUT; break; }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    int st = status;
-#pragma unroll
+    int stt = status;
     for (int j = 0; j < NR; ++j) {
-      if (st == CPM_OK && active[j]) st = CPM_NOT_CONVERGED;
-      a.info->iters[j] = iters[j];
-      a.info->resid[j] = resid[j];
+      if (stt == CPM_OK && (st.active[j] || st.unconv[j])) stt = CPM_NOT_CONVERGED;
+      a.info->iters[j] = st.iters[j];
+      a.info->resid[j] = st.resid[j];
     }
     a.info->outer = 0;
-    set_status(a.info, st);
+    set_status(a.info, stt);
   } else if (status != CPM_OK && threadIdx.x == 0) {
     set_status(a.info, status);
   }

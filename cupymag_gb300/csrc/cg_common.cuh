@@ -84,6 +84,94 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *part, int &par
   return true;
 }
 
+// ---------------------------------------------------------------- FP64 CG state
+// The scalars of NS systems of the plain FP64 CG (csrc/cg.cu, csrc/stencil.cu), in shared memory: lane j of the
+// first warp keeps system j's.  A division or square root in every thread of a CTA costs the FP64 pipe tens of
+// instructions of ~64 cycles per warp (FIGURES).
+template <int NS>
+struct CG64State {
+  double rho[NS], atol[NS], resid[NS], coef[NS];
+  int active[NS], iters[NS], unconv[NS];
+  int any, bad;
+};
+
+template <int NS>
+__device__ __forceinline__ double cg64_pick(const double (&v)[NS], int j) {
+  double t = v[0];
+#pragma unroll
+  for (int k = 1; k < NS; ++k)
+    if (j == k) t = v[k];
+  return t;
+}
+
+// ||b||^2 and ||r||^2; bnorm (may be NULL) takes ||b||.  Ends with a block barrier, as the two below do.
+template <int NS>
+__device__ __forceinline__ void cg64_init(CG64State<NS> &s, const double (&bb)[NS], const double (&rr)[NS], double tol,
+                                          double *bnorm) {
+  if (threadIdx.x < kWarp) {
+    const int j = threadIdx.x < NS ? threadIdx.x : NS - 1;
+    const double bn = sqrt(cg64_pick<NS>(bb, j)), r2 = cg64_pick<NS>(rr, j);
+    const bool act = bn != 0.0;
+    if (threadIdx.x < NS) {
+      s.atol[j] = tol * bn;
+      s.rho[j] = r2;
+      s.resid[j] = sqrt(r2);
+      s.coef[j] = 0.0;
+      s.active[j] = act;
+      s.iters[j] = s.unconv[j] = 0;
+      if (bnorm) bnorm[j] = bn;
+    }
+    const int any = __any_sync(0xffffffffu, act);
+    if (threadIdx.x == 0) {
+      s.any = any;
+      s.bad = 0;
+    }
+  }
+  __syncthreads();
+}
+
+// coef = alpha = rho / p.q of the active systems (0 of the others).
+template <int NS>
+__device__ __forceinline__ void cg64_alpha(CG64State<NS> &s, const double (&pq)[NS]) {
+  if (threadIdx.x < kWarp) {
+    const int j = threadIdx.x < NS ? threadIdx.x : NS - 1;
+    const bool act = s.active[j] != 0;
+    const double al = act ? s.rho[j] / cg64_pick<NS>(pq, j) : 0.0;
+    const int bad = __any_sync(0xffffffffu, act && !isfinite(al));
+    if (threadIdx.x < NS) s.coef[j] = al;
+    if (threadIdx.x == 0) s.bad = bad;
+  }
+  __syncthreads();
+}
+
+// After r.r: the iteration's count and test, coef = beta.  maxiter ends a system unconverged.
+template <int NS>
+__device__ __forceinline__ void cg64_beta(CG64State<NS> &s, const double (&rr)[NS], int maxiter) {
+  if (threadIdx.x < kWarp) {
+    const int j = threadIdx.x < NS ? threadIdx.x : NS - 1;
+    bool act = s.active[j] != 0;
+    const double r2 = cg64_pick<NS>(rr, j), res = sqrt(r2), be = act ? r2 / s.rho[j] : 0.0;
+    const int it = s.iters[j] + 1, bad = __any_sync(0xffffffffu, act && !isfinite(r2));
+    const bool conv = res <= s.atol[j], stop = !conv && it >= maxiter;
+    __syncwarp();  // every lane has read its system
+    if (act && threadIdx.x < NS) {
+      s.iters[j] = it;
+      s.rho[j] = r2;
+      s.resid[j] = res;
+      s.active[j] = !conv && !stop;
+      s.unconv[j] = stop;
+    }
+    act = act && !conv && !stop;
+    const int any = __any_sync(0xffffffffu, act);
+    if (threadIdx.x < NS) s.coef[j] = be;
+    if (threadIdx.x == 0) {
+      s.bad = bad;
+      s.any = any;
+    }
+  }
+  __syncthreads();
+}
+
 // ---------------------------------------------------------------- reliable-update CG state
 // State of one system of the FP32 CG with lagged FP64 reliable updates
 // (csrc/cg.cu, csrc/stencil.cu, csrc/batched.cu).  The transitions below are the whole

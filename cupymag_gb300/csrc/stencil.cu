@@ -54,6 +54,8 @@ struct StencilCG {
   float *xh, *xl;     // x split into floats hi + lo for double-float residual passes (null: FP64 only)
   df::DF cdf[27];     // the scalar coefficients as double-float values
   double df_err;      // error bound of a double-float residual as a multiple of ||b|| (<= 0: off)
+  int even;           // FP64 CG on an elastic stencil even in the offset: products over pairs (even3_rows)
+  double e64[9 * 14];
 };
 
 // Number of independent systems (each with its own CG scalars).
@@ -69,6 +71,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
   constexpr int U = NC * NR;
   constexpr int NS = n_systems<NC, NR>();
   __shared__ double s_red[2 * 3][kCGWarps];
+  __shared__ CG64State<NS> st;
   const int64_t n = a.S.n;
   const int64_t d0 = min(n, (int64_t)blockIdx.x * a.dofs_per_cta);
   const int64_t d1 = min(n, d0 + a.dofs_per_cta);
@@ -98,25 +101,19 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
     set_status(a.info, CPM_BARRIER_TIMEOUT);
     return;
   }
-  double atol[NS], rho[NS], resid[NS];
-  int active[NS], iters[NS];
-  bool any = false;
+  double bb[NS], rr0[NS];
 #pragma unroll
   for (int j = 0; j < NS; ++j) {
-    const double bn = sqrt(v[j]);
-    atol[j] = a.tol * bn;
-    rho[j] = v[NS + j];
-    resid[j] = sqrt(v[NS + j]);
-    active[j] = bn != 0.0;
-    iters[j] = 0;
-    any |= active[j] != 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.info->bnorm[j] = bn;
+    bb[j] = v[j];
+    rr0[j] = v[NS + j];
   }
+  cg64_init<NS>(st, bb, rr0, a.tol, blockIdx.x == 0 ? a.info->bnorm : nullptr);
+  bool any = st.any != 0;
   if (use_init) {
     for (int64_t dof = d0 + threadIdx.x; dof < d1; dof += kCGThreads)
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (!active[sys_of<NC, NR>(u)]) a.x[uidx<NC, NR>(n, dof, u)] = a.b[uidx<NC, NR>(n, dof, u)];
+        if (!st.active[sys_of<NC, NR>(u)]) a.x[uidx<NC, NR>(n, dof, u)] = a.b[uidx<NC, NR>(n, dof, u)];
   }
   int status = CPM_OK;
   for (int k = 0; any && k < a.maxiter; ++k) {
@@ -126,7 +123,12 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
     for (int j = 0; j < NS; ++j) pq[j] = 0.0;
     for (int64_t dof = d0 + threadIdx.x; dof < d1; dof += kCGThreads) {
       double y[U];
-      apply<double, NC, NR>(a.S, a.p, (int)dof, y);
+      if constexpr (NC == 3) {
+        if (a.even && !(a.S.flags && a.S.flags[dof])) even3_rows(a.S, a.e64, a.p, (int)dof, y);
+        else apply<double, NC, NR>(a.S, a.p, (int)dof, y);
+      } else {
+        apply<double, NC, NR>(a.S, a.p, (int)dof, y);
+      }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int64_t i = uidx<NC, NR>(n, dof, u);
@@ -135,14 +137,15 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
       }
     }
     if (!grid_sum<NS>(pq, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    cg64_alpha<NS>(st, pq);
+    if (st.bad) { status = CPM_NONFINITE; break; }
     double alpha[NS];
-    bool bad = false;
+    int active[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
-      alpha[j] = active[j] ? rho[j] / pq[j] : 0.0;
-      if (active[j] && !isfinite(alpha[j])) bad = true;
+      alpha[j] = st.coef[j];
+      active[j] = st.active[j];
     }
-    if (bad) { status = CPM_NONFINITE; break; }
     double rr[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) rr[j] = 0.0;
@@ -159,22 +162,16 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
       }
     }
     if (!grid_sum<NS>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
-    any = false;
+    cg64_beta<NS>(st, rr, a.maxiter);
+    if (st.bad) { status = CPM_NONFINITE; break; }
+    any = st.any != 0;
+    if (!any) break;
     double beta[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
-      beta[j] = 0.0;
-      if (!active[j]) continue;
-      if (!isfinite(rr[j])) bad = true;
-      iters[j] += 1;
-      beta[j] = rr[j] / rho[j];
-      rho[j] = rr[j];
-      resid[j] = sqrt(rr[j]);
-      if (resid[j] <= atol[j]) active[j] = 0;
-      any |= active[j] != 0;
+      beta[j] = st.coef[j];
+      active[j] = st.active[j];
     }
-    if (bad) { status = CPM_NONFINITE; break; }
-    if (!any || k + 1 >= a.maxiter) break;
     for (int64_t dof = d0 + threadIdx.x; dof < d1; dof += kCGThreads) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -186,15 +183,14 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    int st = status;
-#pragma unroll
+    int stt = status;
     for (int j = 0; j < NS; ++j) {
-      if (st == CPM_OK && active[j]) st = CPM_NOT_CONVERGED;
-      a.info->iters[j] = iters[j];
-      a.info->resid[j] = resid[j];
+      if (stt == CPM_OK && (st.active[j] || st.unconv[j])) stt = CPM_NOT_CONVERGED;
+      a.info->iters[j] = st.iters[j];
+      a.info->resid[j] = st.resid[j];
     }
     a.info->outer = 0;
-    set_status(a.info, st);
+    set_status(a.info, stt);
   } else if (status != CPM_OK && threadIdx.x == 0) {
     set_status(a.info, status);
   }
@@ -1091,6 +1087,7 @@ static int launch_stencil_cg(const cpm_stencil *s, const double *b, double *x, c
       }
     }
   }
+  if (fp64 && NC == 3) a.even = even3_coefs(s->coef, a.e64);
   if constexpr (NC == 1) {
     if (!fp64) {
       a.quads = quads_ok(s) && ((uintptr_t)x & 15) == 0 ? 1 : 0;
