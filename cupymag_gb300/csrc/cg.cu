@@ -79,10 +79,13 @@ __device__ __forceinline__ void row_range(const IT *rp, int64_t row, int64_t &s,
 // FP64 pipes of GB300 can sustain at HBM speed.
 template <int NR, typename IT>
 __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
-  __shared__ double s_red[2 * NR][kCGWarps];
   __shared__ CG64State<NR> st;
   extern __shared__ __align__(16) unsigned char s_tile[];
   const TileSmem tile = tile_smem(s_tile);
+  // the reductions stage their values where the tiles were (tile_rows ends with a block barrier; a fifth CTA fits an SM that way: 131 -> 126 us per
+  // iteration of the 48^3 elastic solve)
+  static_assert(sizeof(double) * 2 * NR * kCGThreads <= kTileSmemBytes, "reductions fit the tile");
+  double(*s_red)[kCGThreads] = reinterpret_cast<double(*)[kCGThreads]>(s_tile);
   const int G = a.group;
   const int R = kCGThreads / G;
   const bool lead = (threadIdx.x % G) == 0;
@@ -126,7 +129,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
       }
     }
   }
-  if (!grid_sum<2 * NR>(v, a.part, par, a.bar, tns, s_red)) {
+  if (!grid_sum_wide<2 * NR>(v, a.part, par, a.bar, tns, s_red)) {
     set_status(a.info, CPM_BARRIER_TIMEOUT);
     return;
   }
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
         }
       }
     }
-    if (!grid_sum<NR>(pq, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    if (!grid_sum_wide<NR>(pq, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
     cg64_alpha<NR>(st, pq);
     if (st.bad) { status = CPM_NONFINITE; break; }
     double alpha[NR];
@@ -190,7 +193,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
         rr[j] = fma(rn, rn, rr[j]);
       }
     }
-    if (!grid_sum<NR>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    if (!grid_sum_wide<NR>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
     cg64_beta<NR>(st, rr, a.maxiter);
     if (st.bad) { status = CPM_NONFINITE; break; }
     any = st.any != 0;
@@ -245,7 +248,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
 // against 668 us in place).  The CG state lives in shared memory (IRState).
 template <int NR, typename IT>
 __global__ void __launch_bounds__(kCGThreads) cg_ir_kernel(CGArgs<NR, IT> a) {
-  __shared__ double s_red[9][kCGWarps];
+  __shared__ double s_red[3 * NR][kCGThreads];
   __shared__ IRState st[NR];
   __shared__ float s_ab[NR];
   __shared__ int s_mask[3];  // active, need, status
@@ -296,7 +299,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_ir_kernel(CGArgs<NR, IT> a) {
       }
     }
   }
-  if (!grid_sum<2 * NR>(v, a.part, par, a.bar, tns, s_red)) {
+  if (!grid_sum_wide<2 * NR>(v, a.part, par, a.bar, tns, s_red)) {
     set_status(a.info, CPM_BARRIER_TIMEOUT);
     return;
   }
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_ir_kernel(CGArgs<NR, IT> a) {
       }
     }
     // t.t and t.p only on an iteration with a pending update (FP64 adds are slow on GB300)
-    if (!grid_sum<3 * NR>(pt, a.part, par, a.bar, tns, s_red, needm ? 3 * NR : NR)) {
+    if (!grid_sum_wide<3 * NR>(pt, a.part, par, a.bar, tns, s_red, needm ? 3 * NR : NR)) {
       status = CPM_BARRIER_TIMEOUT;
       break;
     }
@@ -403,7 +406,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_ir_kernel(CGArgs<NR, IT> a) {
     double rr[NR];
 #pragma unroll
     for (int j = 0; j < NR; ++j) rr[j] = (double)rrf[j];
-    if (!grid_sum<NR>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    if (!grid_sum_wide<NR>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
     if (threadIdx.x == 0) {
       int nm = 0, bad = 0;
       for (int j = 0; j < NR; ++j) {
@@ -515,8 +518,11 @@ static int launch_cg(const cpm_csr *A, const double *b, double *x, const cpm_cg_
   a.group = group_size(maxrow, kCGThreads);
   int64_t gmax = (int64_t)occ * sm_count();
   if (gmax > kMaxGrid) gmax = kMaxGrid;
-  // at least ~64 rows per CTA so small systems do not pay for idle CTAs at barriers
-  int64_t G = (a.n + 63) / 64;
+  // Small systems: at least 64 rows per CTA, 128 from 16 k rows on (fewer barrier arrivals and partials).  Measured on
+  // GB300, FP64, us per iteration at 64 / 128: demag 16^3 13.8 / 14.2, 32^3 17.4 / 15.8, three right-hand sides
+  // 32^3 32.2 / 27.5; elastic rows (81 entries) gain from the smaller blocks at 16^3 (18.6 / 24.2).
+  const int64_t least = a.n >= 16384 && maxrow <= 32 ? 128 : 64;
+  int64_t G = (a.n + least - 1) / least;
   if (G > gmax) G = gmax;
   if (G < 1) G = 1;
   int64_t rpc = (a.n + G - 1) / G;

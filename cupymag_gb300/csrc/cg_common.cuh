@@ -84,10 +84,59 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *part, int &par
   return true;
 }
 
+// grid_sum with a warp per value: every value is staged at once (s: NV rows of the CTA's kCGThreads threads), warp j
+// adds value j's, and after the barrier value j's partials of all CTAs, each in grid_sum's order (the same bits).  Six
+// block barriers for any NV, where grid_sum takes 2 + 6 NV with the other warps idle.  Measured on GB300: the plain
+// FP64 step at 32^3 on CSR operators 5.3 -> 4.4 ms (three right-hand sides 32 -> 24 us per iteration); one warp loading
+// all partials instead of every thread made it slower than grid_sum (19 against 13.6 us per tet iteration).
+template <int NV>
+__device__ __forceinline__ bool grid_sum_wide(double (&v)[NV], double *part, int &parity, GridBarrier *bar,
+                                              unsigned long long tns, double (*s)[kCGThreads], int nv = NV) {
+  const int G = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  part += (size_t)parity * kPartHalf;
+  parity ^= 1;
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+    if (j < nv) s[j][threadIdx.x] = v[j];
+  __syncthreads();
+  for (int j = warp; j < nv; j += kCGWarps) {
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < kCGWarps; ++k) t += s[j][k * kWarp + lane];
+    t = warp_sum(t);
+    if (lane == 0) part[(size_t)blockIdx.x * NV + j] = t;
+  }
+  if (!grid_sync(bar, G, tns)) return false;
+  double acc[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) acc[j] = 0.0;
+  for (int g = threadIdx.x; g < G; g += kCGThreads)
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (j < nv) acc[j] += __ldcg(&part[(size_t)g * NV + j]);
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+    if (j < nv) s[j][threadIdx.x] = acc[j];
+  __syncthreads();
+  for (int j = warp; j < nv; j += kCGWarps) {
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < kCGWarps; ++k) t += s[j][k * kWarp + lane];
+    t = warp_sum(t);
+    if (lane == 0) s[j][0] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NV; ++j) v[j] = j < nv ? s[j][0] : 0.0;
+  __syncthreads();  // the next staging may overwrite the totals
+  return true;
+}
+
 // ---------------------------------------------------------------- FP64 CG state
 // The scalars of NS systems of the plain FP64 CG (csrc/cg.cu, csrc/stencil.cu), in shared memory: lane j of the
 // first warp keeps system j's.  A division or square root in every thread of a CTA costs the FP64 pipe tens of
-// instructions of ~64 cycles per warp (FIGURES).
+// instructions of ~64 cycles per warp: the plain FP64 step at 32^3 on CSR operators took 7.3 ms that way and 5.3 ms
+// with these.
 template <int NS>
 struct CG64State {
   double rho[NS], atol[NS], resid[NS], coef[NS];

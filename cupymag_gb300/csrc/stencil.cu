@@ -70,7 +70,7 @@ template <int NC, int NR>
 __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __grid_constant__ StencilCG a) {
   constexpr int U = NC * NR;
   constexpr int NS = n_systems<NC, NR>();
-  __shared__ double s_red[2 * 3][kCGWarps];
+  __shared__ double s_red[2 * NS][kCGThreads];
   __shared__ CG64State<NS> st;
   const int64_t n = a.S.n;
   const int64_t d0 = min(n, (int64_t)blockIdx.x * a.dofs_per_cta);
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
       v[NS + sys_of<NC, NR>(u)] = fma(ri, ri, v[NS + sys_of<NC, NR>(u)]);
     }
   }
-  if (!grid_sum<2 * NS>(v, a.part, par, a.bar, tns, s_red)) {
+  if (!grid_sum_wide<2 * NS>(v, a.part, par, a.bar, tns, s_red)) {
     set_status(a.info, CPM_BARRIER_TIMEOUT);
     return;
   }
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
         pq[sys_of<NC, NR>(u)] = fma(a.p[i], y[u], pq[sys_of<NC, NR>(u)]);
       }
     }
-    if (!grid_sum<NS>(pq, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    if (!grid_sum_wide<NS>(pq, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
     cg64_alpha<NS>(st, pq);
     if (st.bad) { status = CPM_NONFINITE; break; }
     double alpha[NS];
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kCGThreads) cg_stencil_fp64_kernel(const __gri
         rr[s] = fma(rn, rn, rr[s]);
       }
     }
-    if (!grid_sum<NS>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    if (!grid_sum_wide<NS>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
     cg64_beta<NS>(st, rr, a.maxiter);
     if (st.bad) { status = CPM_NONFINITE; break; }
     any = st.any != 0;
@@ -241,7 +241,7 @@ __device__ __forceinline__ void cg_stencil_ir_body(const StencilCG &a) {
   constexpr int U = NC * NR;
   constexpr int NS = n_systems<NC, NR>();
   constexpr int TH = kIRThreads;
-  __shared__ double s_red[9][TH / kWarp];
+  __shared__ double s_red[3 * NS][kCGThreads];
   __shared__ IRState st[NS];
   __shared__ float s_ab[NS];
   __shared__ int s_mask[4];  // active, need, error status, double-float pass
@@ -289,7 +289,7 @@ __device__ __forceinline__ void cg_stencil_ir_body(const StencilCG &a) {
       v[NS + s] = fma(ri, ri, v[NS + s]);
     }
   }
-  if (!grid_sum<2 * NS + 1>(v, a.part, par, a.bar, tns, s_red, xh ? 2 * NS + 1 : 2 * NS)) {
+  if (!grid_sum_wide<2 * NS + 1>(v, a.part, par, a.bar, tns, s_red, xh ? 2 * NS + 1 : 2 * NS)) {
     set_status(a.info, CPM_BARRIER_TIMEOUT);
     return;
   }
@@ -421,7 +421,7 @@ __device__ __forceinline__ void cg_stencil_ir_body(const StencilCG &a) {
       }
     }
     // t.t and t.p only on an iteration with a pending update (FP64 adds are slow on GB300)
-    if (!grid_sum<3 * NS>(pt, a.part, par, a.bar, tns, s_red, needm ? 3 * NS : NS)) {
+    if (!grid_sum_wide<3 * NS>(pt, a.part, par, a.bar, tns, s_red, needm ? 3 * NS : NS)) {
       status = CPM_BARRIER_TIMEOUT;
       break;
     }
@@ -468,7 +468,7 @@ __device__ __forceinline__ void cg_stencil_ir_body(const StencilCG &a) {
     double rr[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) rr[j] = (double)rrf[j];
-    if (!grid_sum<NS>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
+    if (!grid_sum_wide<NS>(rr, a.part, par, a.bar, tns, s_red)) { status = CPM_BARRIER_TIMEOUT; break; }
     if (threadIdx.x == 0) {
       int nm = 0, bad = 0, dfall = 1;
       for (int j = 0; j < NS; ++j) {
