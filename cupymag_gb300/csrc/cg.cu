@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(kCGThreads) cg_fp64_kernel(CGArgs<NR, IT> a) {
   __shared__ CG64State<NR> st;
   extern __shared__ __align__(16) unsigned char s_tile[];
   const TileSmem tile = tile_smem(s_tile);
-  // the reductions stage their values where the tiles were (tile_rows ends with a block barrier; a fifth CTA fits an SM that way: 131 -> 126 us per
-  // iteration of the 48^3 elastic solve)
+  // the reductions stage their values where the tiles were (tile_rows ends with a block barrier): a fifth CTA fits
+  // an SM that way, 131 -> 126 us per iteration of the 48^3 elastic solve
   static_assert(sizeof(double) * 2 * NR * kCGThreads <= kTileSmemBytes, "reductions fit the tile");
   double(*s_red)[kCGThreads] = reinterpret_cast<double(*)[kCGThreads]>(s_tile);
   const int G = a.group;

@@ -218,6 +218,57 @@ __device__ __forceinline__ void even3_rows(const Geo &S, const double *e64, cons
   }
 }
 
+// ---------------------------------------------------------------- FP64 products of even scalar stencils
+// The 8 coefficients c[4 |dx| + 2 |dy| + |dz|] of a scalar stencil even along every axis; false unless that is all
+// of it, to 1e-15 of the largest coefficient.
+inline bool even8_coefs(const double *coef, double *c8) {
+  double big = 0.0;
+  for (int e = 0; e < 8; ++e) c8[e] = 0.0;
+  for (int d = 0; d < 27; ++d) {
+    const int m = 4 * (d / 9 != 1) + 2 * ((d / 3) % 3 != 1) + (d % 3 != 1);
+    c8[m] += coef[d] / (double)((m & 4 ? 2 : 1) * (m & 2 ? 2 : 1) * (m & 1 ? 2 : 1));
+    big = coef[d] > big ? coef[d] : -coef[d] > big ? -coef[d] : big;
+  }
+  for (int d = 0; d < 27; ++d) {
+    const double o = coef[d] - c8[4 * (d / 9 != 1) + 2 * ((d / 3) % 3 != 1) + (d % 3 != 1)];
+    if (!(o <= 1e-15 * big && -o <= 1e-15 * big)) return false;
+  }
+  return true;
+}
+
+struct Even8 {
+  double c[8];
+};
+
+// A thread marches along x over planes [x0, x1) at value g of a plane (NR interleaved vectors: NR ny nz values per
+// plane): per plane the sums over y +- 1 and z +- 1 give its parts of the product at its own node and at both x
+// neighbours: 15 FP64 operations per value where the 27-point form takes 27.  emit(i, y) gets the product at plane i.
+template <int NR, typename Emit>
+__device__ __forceinline__ void even8_march(const double (&c)[8], const double *x, int nx, int ny, int nz, int g,
+                                            int x0, int x1, Emit emit) {
+  const int f = g / NR, j = f / nz, k = f - j * nz;
+  const int om = (j == 0 ? (ny - 1) * nz : -nz) * NR, od = (j == ny - 1 ? -(ny - 1) * nz : nz) * NR;
+  const int ol = (k == 0 ? nz - 1 : -1) * NR, orr = (k == nz - 1 ? 1 - nz : 1) * NR;
+  const int64_t plane = (int64_t)ny * nz * NR;
+  double acc = 0.0, side = 0.0;
+  for (int i = x0 - 1; i <= x1; ++i) {
+    const double *p = x + (i < 0 ? nx - 1 : i >= nx ? 0 : i) * plane + g;
+    const double v = p[0], u = p[om] + p[od], t = p[ol] + p[orr];
+    const double w = (p[ol + om] + p[ol + od]) + (p[orr + om] + p[orr + od]);
+    const double s = fma(c[7], w, fma(c[6], u, fma(c[5], t, c[4] * v)));
+    if (i > x0) emit(i - 1, acc + s);
+    if (i >= x0 && i < x1) acc = fma(c[3], w, fma(c[2], u, fma(c[1], t, fma(c[0], v, side))));
+    side = s;
+  }
+}
+
+// Planes per march: 16, fewer while the marches are too few to give each SM 8 warps.
+inline int even8_planes(int nx, int64_t values, int sms) {
+  int lx = 16;
+  while (lx > 2 && values / 32 * ((nx + lx - 1) / lx) < 8ll * sms) lx /= 2;
+  return lx < nx ? lx : nx;
+}
+
 // y at one DOF (all NC*NR components) in T, for x stored as TX.  Rows
 // flagged as unit / empty are handled first; only rows next to an excluded
 // column test neighbour flags.

@@ -1,4 +1,5 @@
-"""The marching derivative kernels (csrc/deriv.cu, mirror_kernel) against the pair kernels."""
+"""The marching FP64 products (csrc/deriv.cu mirror_kernel, csrc/stencil_ops.cuh even8_march) against the forms that
+take any stencil."""
 import numpy as np
 import pytest
 import torch
@@ -53,3 +54,30 @@ def test_marching_products_match_the_pair_kernels(dims):
     a, b = F.spmv(E0), F2.spmv(E0)
     close(a, b, 12 * eel * big(E0), "F_el E0")
     assert float(a[0]) == float(a[n]) == float(a[2 * n]) == 0.0
+
+
+@pytest.mark.parametrize("dims", [(3, 3, 3), (17, 4, 5), (16, 33, 3), (35, 9, 31), (5, 40, 64)])
+@pytest.mark.parametrize("nvec", [1, 3])
+def test_marching_scalar_product_matches_the_per_node_form(dims, nvec):
+    """Identity, empty and excluded rows among the flags; planes that the marches split unevenly.  One coefficient
+    moved by 1e-13 of the largest keeps the per-node form: at most 1e-13 max|c| max|x| per output apart from
+    rounding (27 terms)."""
+    from cupymag_gb300.core.assemble_simulation_operators import SimulationOperators
+    from cupymag_gb300.utils.stencil_operator import COL_EXCLUDED, ROW_IDENTITY, ROW_ZERO, StencilOperator
+    from cupymag_gb300.workloads import hex_params
+    so = SimulationOperators(hex_params(6, 1, False, False), device="cuda").stencil_operators()
+    rng = np.random.default_rng(sum(dims) + nvec)
+    n = dims[0] * dims[1] * dims[2]
+    flags = np.zeros(n, dtype=np.uint8)
+    flags[rng.integers(0, n, 3)] = ROW_IDENTITY | COL_EXCLUDED
+    flags[rng.integers(0, n, 2)] = ROW_ZERO
+    x = torch.as_tensor(rng.normal(size=(n, nvec) if nvec == 3 else n), device="cuda")
+    for name in ("F1", "A1", "A_demag"):
+        c = so[name].coef_host
+        moved = c.copy()
+        moved[5] += 1e-13 * np.abs(c).max()
+        a = StencilOperator(*dims, c, flags).spmv(x, alpha=-2.0)
+        b = StencilOperator(*dims, moved, flags).spmv(x, alpha=-2.0)
+        big = float(x.abs().max())
+        bound = 2 * (1e-13 * np.abs(c).max() + 54 * 2.0 ** -53 * np.abs(c).sum()) * big
+        assert float((a - b).abs().max()) <= bound, name
