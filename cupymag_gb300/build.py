@@ -4,7 +4,8 @@ Each translation unit under ``csrc/`` is compiled in parallel for
 ``-gencode arch=compute_103a,code=sm_103a`` and linked into a shared library
 that exports the C-ABI declared in ``include/cupymag_gb300.h``.  The element-wise
 LLG kernels are compiled without FMA contraction so their rounding follows the
-reference's separately-rounded array operations.
+reference's separately-rounded array operations (its matrix products, BLAS calls,
+are explicit FMAs there).
 
 Usage: ``python -m cupymag_gb300.build [--force]``.
 """
