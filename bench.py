@@ -3,7 +3,7 @@
 Default workload: 128^3 hex with magnetoelastic coupling and the [111]
 rotation (cfg "hex128_me"), in the precision form on the matrix-free stencil
 operators: the elastic and demag solves by FFT inside FP64 refinement, the
-Gauss-Seidel solves by FP32 CG with FP64 reliable updates.  A "step" is one
+Gauss-Seidel solves by FP32 Chebyshev cycles with true residuals between them.  A "step" is one
 Gauss-Seidel-projection LLG step at the next field of the 500-step sweep,
 with all operators and state resident in HBM.
 

@@ -26,8 +26,10 @@ import numpy as np
 import torch
 
 
-def _bytes(op, nrhs, iters, outer, fp32, csr):
+def _bytes(op, nrhs, iters, outer, fp32, csr, cheb=False):
     u = op.shape[0] * nrhs
+    if cheb:  # 16 B per step, 12 start, 20 per true residual, 8 FP32 check, 16 solution (csrc/cheby.cuh)
+        return u * (16 * max(iters - 1, 0) + 36 + 20 * outer)
     if not csr:
         return u * (44 * iters + 48 * max(outer, 1)) if fp32 else u * (88 * iters + 24)
     ip = op.indptr.element_size()
@@ -194,7 +196,8 @@ def main(argv=None):
     d = infos[-1]
     its = max(d["iters"][:nrhs])
     ms = float(np.median(times))
-    nb = _bytes(op, nrhs, its, d["outer"], args.precision == "IR", csr) * args.batch
+    cheb = not csr and args.precision == "IR" and args.op in ("A1", "A2") and args.form == 0 and not args.precond
+    nb = _bytes(op, nrhs, its, d["outer"], args.precision == "IR", csr, cheb) * args.batch
     print(json.dumps({"op": args.op, "edge": args.edge, "n": n, "nrhs": nrhs, "precision": args.precision,
                       "inner_tol": inner_tol, "form": args.form, "precond": args.precond,
                       "fft_layout": args.fft_layout if args.precond else None,

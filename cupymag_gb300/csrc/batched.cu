@@ -17,6 +17,9 @@
 // ends when a device counter of systems that are still iterating drops to
 // zero.  Every wait is bounded (GridBarrier).
 //
+// Scalar systems in precision 1 that the Chebyshev rule takes (csrc/cheby.cuh) run in a launch of their own before
+// these kernels, which serve the rest.
+//
 // Precision 0 is the three-phase FP64 CG of csrc/stencil.cu.  Precision 1 is
 // FP32 CG with FP64 reliable updates in a form that needs no extra barrier:
 // when the FP32 recursive residual has fallen by inner_tol (or below the

@@ -17,7 +17,7 @@
 // barrier, where a CG iteration moves 44 bytes through three barriers and two
 // grid reductions.  The number of steps of a cycle follows from the reduction
 // it needs, ||r_k|| <= ||r_0|| / T_k; A1 and A2 (condition numbers 10.5 and
-// 23.3) take 40 and 61 steps from a cold start to tol 1e-10, CG 28-36 and 41-55.
+// 23.3) take 40 and 60 steps from a cold start to tol 1e-10, CG 28-36 and 41-55.
 // Measured on GB300, us per cold solve, CG / this: A1 x 3 at 128^3 3500 / 960,
 // at 112 x 96 x 90 3790 / 578; A2 x 3 at 128^3 5000 / 1350; A1 at 20^3 490 /
 // 244 through solve_cg.  A 128^3 x 3 step takes 18.6 us (18.7 bytes per unknown

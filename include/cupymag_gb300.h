@@ -204,7 +204,7 @@ size_t cpm_cg_stencil_workspace_bytes(int64_t unknowns, int nrhs, int precision)
  * number at most 64, runs Chebyshev steps between its true residuals in place of CG: on the free DOFs the
  * operator's spectrum lies between the symbol's extremes, so the steps need no inner products (one grid
  * barrier and 16 bytes per unknown each).  Same stopping test and statuses; info->iters counts the steps
- * (40 and 61 where CG takes 28-36 and 41-55 on A1 and A2).  maxiter below four times a cold start's
+ * (40 and 60 where CG takes 28-36 and 41-55 on A1 and A2).  maxiter below four times a cold start's
  * steps, and flagged rows that are not pinned, keep CG. */
 size_t cpm_cg_stencil_workspace(const cpm_stencil *S, int nrhs, int precision);
 /* The bound behind that choice, as a multiple of ||b||: 2 g sum|c| / sigma_min with g = 128 * 2^-48 and
