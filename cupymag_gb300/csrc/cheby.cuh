@@ -616,7 +616,7 @@ __device__ __noinline__ void cheb_start(const ChebSys &S, int l, bool use_init, 
 
 // Returns false (in every thread of the system's CTAs, before x is written) when the system is not one
 // for this iteration: a flagged row that is not pinned, or a right-hand side or warm start that is not
-// finite in floats.
+// finite in floats.  Other CTAs may then still read S.part: its next user needs a barrier (or a launch) in front.
 template <int NR>
 __device__ __forceinline__ bool cheb_solve(const ChebSys &S, const ChebOp &op, int l, double (*sred)[kCGWarps]) {
   __shared__ ChebState<NR> st;  // thread 0 writes it after each reduction (FP64 scalars are slow in every thread)

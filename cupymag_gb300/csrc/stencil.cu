@@ -541,7 +541,8 @@ __global__ void __launch_bounds__(kIRThreads, 4) cg_stencil_ir_kernel(const __gr
 // ---------------------------------------------------------------- Chebyshev iteration (csrc/cheby.cuh)
 // The default of the FP32 form for the scalar stencils that cheb_operator accepts.  A system that turns
 // out not to fit on the device (a flagged row that is not pinned, values that are not finite in floats) is
-// solved by the CG above in the same launch.
+// solved by the CG above in the same launch, behind a barrier of its own: the CG starts over in the partials that
+// slower CTAs may still be summing.
 struct ChebSolve {
   ChebSys sys;
   ChebOp op;
@@ -551,7 +552,12 @@ struct ChebSolve {
 template <int NR>
 __global__ void __launch_bounds__(kChebThreads, kChebBlocks) cheb_stencil_kernel(const __grid_constant__ ChebSolve a) {
   __shared__ double s_red[NR + 1][kCGWarps];
-  if (!cheb_solve<NR>(a.sys, a.op, blockIdx.x, s_red)) cg_stencil_ir_body<1, NR>(a.cg);
+  if (cheb_solve<NR>(a.sys, a.op, blockIdx.x, s_red)) return;
+  if (!grid_sync(a.sys.bar, a.sys.ncta, a.op.timeout_ns)) {
+    set_status(a.cg.info, CPM_BARRIER_TIMEOUT);
+    return;
+  }
+  cg_stencil_ir_body<1, NR>(a.cg);
 }
 
 // ---------------------------------------------------------------- FP32 CG with two grid barriers per iteration

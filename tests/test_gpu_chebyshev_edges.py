@@ -1,0 +1,79 @@
+"""Where the Chebyshev iteration of the projection solves hands over, decides and ends."""
+import numpy as np
+import pytest
+import torch
+
+from . import _golden as G
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+
+
+def _case(dims, defect):
+    from cupymag_gb300.core.assemble_simulation_operators import SimulationOperators
+    p = G.params(G.load("hex_me_rot")).with_(Nx=dims[0], Ny=dims[1], Nz=dims[2], Ndx=defect, Ndy=defect, Ndz=defect)
+    S = SimulationOperators(p)
+    return S, S.stencil_operators(), S.host_operators()
+
+
+def _solve(op, b, x0=None, form=0, maxiter=20000, tol=TOL, solver=None):
+    from cupymag_gb300.solvers.linear_solvers import CGSolver, decode_info, new_info
+    bd = torch.as_tensor(b, device="cuda").contiguous()
+    x = torch.zeros_like(bd) if x0 is None else torch.as_tensor(x0, device="cuda").clone().contiguous()
+    info = new_info(1)
+    (solver or CGSolver()).launch(op, bd, x, info[0], tol=tol, maxiter=maxiter, precision="IR", inner_tol=1e-5,
+                                  form=form, use_init=x0 is not None)
+    return x.cpu().numpy(), decode_info(info[0].cpu().numpy())
+
+
+@pytest.mark.parametrize("nrhs", [1, 3])
+@pytest.mark.parametrize("dims", [(5, 4, 3), (12, 13, 14), (40, 33, 37)])
+def test_hand_over_to_cg_gives_the_same_bits_every_time(dims, nrhs):
+    """Systems with a flagged row that is not pinned run CG behind the Chebyshev start of the same launch: the
+    stopping test holds and every repetition gives the same bits and the same record."""
+    from cupymag_gb300.solvers.linear_solvers import CGSolver
+    from cupymag_gb300.utils.stencil_operator import COL_EXCLUDED, ROW_IDENTITY, StencilOperator
+    op = _case(dims, 0)[1]["A1"]
+    f = np.zeros(op.n, dtype=np.uint8)
+    f[17] = ROW_IDENTITY                       # its column stays in the other rows
+    f[41] = ROW_IDENTITY | COL_EXCLUDED
+    odd = StencilOperator(*dims, op.coef_host, f)
+    rng = np.random.default_rng(8)
+    b = rng.normal(size=(op.n, 3) if nrhs == 3 else op.n)
+    b[17] = 0.0
+    solver = CGSolver()
+    for x0 in (None, 0.1 * rng.normal(size=b.shape)):
+        if x0 is not None:
+            x0[17] = 0.0
+        x, inf = _solve(odd, b, x0, solver=solver)
+        assert inf["status"] == 0, inf
+        r = b - odd.spmv(torch.as_tensor(x, device="cuda")).cpu().numpy()
+        assert np.all(np.linalg.norm(r.reshape(op.n, -1), axis=0) <=
+                      1.001 * TOL * np.linalg.norm(b.reshape(op.n, -1), axis=0))
+        for _ in range(40):
+            y, other = _solve(odd, b, x0, solver=solver)
+            assert np.array_equal(x, y) and inf == other
+
+
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_values_beyond_floats_end_as_in_cg(nrhs):
+    """A warm start or a right-hand side that is not finite in floats: the status is the CG form's, and the next
+    solve on the same workspace is sound."""
+    from cupymag_gb300 import _native as N
+    from cupymag_gb300.solvers.linear_solvers import CGSolver
+    op = _case((9, 8, 10), 2)[1]["A2"]
+    rng = np.random.default_rng(2)
+    b = rng.normal(size=(op.n, 3) if nrhs == 3 else op.n)
+    x0 = np.zeros_like(b)
+    x0[5] = 1e200
+    bad = b.copy()
+    bad[3] = np.inf
+    solver = CGSolver()
+    ref, good = _solve(op, b, solver=solver)
+    assert good["status"] == 0
+    for rhs, start in ((b, x0), (bad, None)):
+        _, inf = _solve(op, rhs, start, solver=solver)
+        _, cg = _solve(op, rhs, start, form=N.CG_FORM_THREE_BARRIER)
+        assert inf["status"] == cg["status"] != 0, (inf, cg)
+        again, inf = _solve(op, b, solver=solver)
+        assert np.array_equal(again, ref) and inf == good
