@@ -838,23 +838,22 @@ template <int NR>
 __global__ void __launch_bounds__(128) stencil_march_kernel(const __grid_constant__ StencilOp S,
                                                             const __grid_constant__ Even8 e, const double *x,
                                                             double *y, double alpha, int lx) {
-  const int g = blockIdx.x * 128 + threadIdx.x, values = S.ny * S.nz * NR;
-  if (g >= values) return;
+  const int nyz = S.ny * S.nz, values = nyz * NR;
+  const unsigned gu = blockIdx.x * 128u + threadIdx.x;  // the last block may end beyond 2^31
+  if (gu >= (unsigned)values) return;
+  const int g = (int)gu, f = g / NR;
   const int x0 = blockIdx.y * lx, x1 = min(S.nx, x0 + lx);
   const uint8_t *flags = S.flags;
   even8_march<NR>(e.c, x, S.nx, S.ny, S.nz, g, x0, x1, [&](int i, double v) {
-    const int64_t o = (int64_t)i * values + g;
-    if (flags) {
-      const int dof = (int)((unsigned)o / NR);
-      if (flags[dof]) {
-        double t[NR];
-        apply<double, 1, NR>(S, x, dof, t);
+    const int dof = i * nyz + f;  // below 2^31; value indices need 64 bits (up to 3 x 2^31)
+    if (flags && flags[dof]) {
+      double t[NR];
+      apply<double, 1, NR>(S, x, dof, t);
 #pragma unroll
-        for (int r = 0; r < NR; ++r)
-          if ((int)(g % NR) == r) v = t[r];
-      }
+      for (int r = 0; r < NR; ++r)
+        if (g - f * NR == r) v = t[r];
     }
-    y[o] = alpha * v;
+    y[(int64_t)i * values + g] = alpha * v;
   });
 }
 

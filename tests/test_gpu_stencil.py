@@ -291,3 +291,41 @@ def test_double_float_residuals_keep_the_fp64_stopping_test(dims, nrhs):
                 assert idf["df_updates"] == 0 and np.array_equal(xdf, x64), name
             else:
                 assert idf["df_updates"] >= 1, (name, idf)
+
+
+def test_product_of_three_vectors_finds_the_flags_beyond_2_32_values():
+    """1.44e9 nodes with three vectors are 4.3e9 values: a unit row whose value indices need more than 32 bits gives
+    x, and the row at the index cut to 32 bits stays an ordinary one (the rows' sums on a constant and a marked x)."""
+    from cupymag_gb300.utils.stencil_operator import COL_EXCLUDED, NEAR_EXCLUDED, ROW_IDENTITY, StencilOperator
+    dims = (1500, 980, 980)
+    n = dims[0] * dims[1] * dims[2]
+    free, _ = torch.cuda.mem_get_info()
+    if free < 2 * 24 * n + n + (8 << 30):
+        pytest.skip("needs about 80 GB of device memory")
+    rng = np.random.default_rng(4)
+    c8 = rng.uniform(0.1, 1.0, size=8)
+    coef = np.array([c8[4 * (d // 9 != 1) + 2 * (d // 3 % 3 != 1) + (d % 3 != 1)] for d in range(27)])
+    op = StencilOperator(*dims, coef)
+    row = n - 7 * dims[1] * dims[2] - 5 * dims[2] - 11
+    cut = (3 * row % 2 ** 32) // 3
+    assert 3 * row >= 2 ** 32 and cut < n
+    op.flags = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    i, j, k = row // (dims[1] * dims[2]), row // dims[2] % dims[1], row % dims[2]
+    near = [(((i + a) * dims[1]) + j + b) * dims[2] + k + c for a in (-1, 0, 1) for b in (-1, 0, 1) for c in (-1, 0, 1)]
+    op.flags[torch.tensor(near, device="cuda")] = NEAR_EXCLUDED
+    op.flags[row] = ROW_IDENTITY | COL_EXCLUDED | NEAR_EXCLUDED
+    x = torch.ones((n, 3), dtype=torch.float64, device="cuda")
+    mark = torch.tensor([2.0, 3.0, 5.0], dtype=torch.float64, device="cuda")
+    x[row] = mark
+    y = torch.empty_like(x)
+    try:
+        op.spmv(x, out=y)
+        assert torch.equal(y[row], mark)
+        tol = 64 * 2.0 ** -53 * coef.sum()
+        assert (y[cut] - coef.sum()).abs().max() <= tol
+        for q, d in zip(near, range(27)):
+            if d != 13:   # the unit row's column is left out (offset of `row` from `q`: -d)
+                assert (y[q] - (coef.sum() - coef[26 - d])).abs().max() <= tol, d
+    finally:
+        del x, y
+        torch.cuda.empty_cache()
