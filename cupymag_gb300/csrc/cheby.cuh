@@ -556,11 +556,11 @@ struct ChebState {
 };
 
 // Steps of the next cycle, enough for every pending right-hand side, and whether its end may be proven by an
-// FP32 residual.
+// FP32 residual (not where the caller asked for FP64 residuals).
 template <int NR>
 __device__ __forceinline__ int cheb_cycle(ChebState<NR> &st, const ChebSys &S, const ChebOp &op, int iters) {
   int steps = 2;
-  st.check = 1;
+  st.check = op.df;
   for (int s = 0; s < NR; ++s) {
     if (!((st.pending >> s) & 1)) continue;
     const double goal = kChebAim * S.tol * st.bn[s];

@@ -77,3 +77,28 @@ def test_values_beyond_floats_end_as_in_cg(nrhs):
         assert inf["status"] == cg["status"] != 0, (inf, cg)
         again, inf = _solve(op, b, solver=solver)
         assert np.array_equal(again, ref) and inf == good
+
+
+@pytest.mark.parametrize("name", ["A1", "A2"])
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_fp64_residuals_decide_where_they_are_asked_for(name, nrhs):
+    """df_residual = False: every cycle of a cold solve ends with an FP64 residual of the x that is returned (the
+    default form proves the last one in FP32).  The residual reported is then that of x to the rounding of an FP64
+    product, 64 * 2^-53 sum|c| ||x||, relative to a residual near tol ||b||."""
+    from cupymag_gb300.solvers.linear_solvers import CGSolver
+    S, so, csr = _case((12, 11, 13), 3)
+    A, op = csr[name], so[name]
+    rng = np.random.default_rng(7)
+    b = rng.normal(size=(op.n, 3) if nrhs == 3 else op.n)
+    solver = CGSolver()
+    _, fast = _solve(op, b, solver=solver)
+    solver.df_residual = False
+    x, inf = _solve(op, b, solver=solver)
+    assert inf["status"] == 0 and inf["df_updates"] == 0 and fast["df_updates"] == fast["outer"] >= 1
+    assert inf["iters"] == fast["iters"] and inf["outer"] == fast["outer"] + 1, (inf, fast)
+    bb, xx = b.reshape(op.n, -1), x.reshape(op.n, -1)
+    for r in range(nrhs):
+        res = np.linalg.norm(bb[:, r] - A @ xx[:, r])
+        tol = 64 * 2.0 ** -53 * np.abs(op.coef_host).sum() * np.linalg.norm(xx[:, r])
+        assert res <= TOL * np.linalg.norm(bb[:, r])
+        assert abs(inf["resid"][r] - res) <= tol, (inf["resid"][r], res, tol)
