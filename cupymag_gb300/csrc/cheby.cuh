@@ -288,7 +288,7 @@ __device__ __forceinline__ void cheb_plane(const ChebQuad &c, const f32x2 (&co)[
 
 // out = ca x + cb out + cg r - ch A x on the free DOFs, 0 on the pinned ones (out is not read where cb = 0), with ca
 // and ch inside the coefficients.  CHECK: nothing is written; the chunk partials of |out|^2 times scale^2 per
-// right-hand side go to `half` (cb = 0).
+// right-hand side go to `half` (cb = 0): the squares of a quad are added in FP32 (5 roundings), the quads in FP64.
 template <int NR, bool CHECK>
 __device__ __forceinline__ void cheb_pass(const ChebSys &S, const ChebOp &op, int l, const float *x, float *out,
                                           const float *r, float ca, float cb, float cg, float ch,
@@ -307,7 +307,7 @@ __device__ __forceinline__ void cheb_pass(const ChebSys &S, const ChebOp &op, in
   for (int chunk = l; chunk < chunks; chunk += S.ncta) {
     const int tile = chunk / ranges, x0 = (chunk - tile * ranges) * lx, x1 = min(nx, x0 + lx);
     const int run = tile * S.tw + warp;
-    float sum = 0.0f;
+    double sum = 0.0;
     int rhs = 0;
     if (warp < S.tw && run < S.runs) {
       ChebQuad c;
@@ -384,7 +384,7 @@ __device__ __forceinline__ void cheb_pass(const ChebSys &S, const ChebOp &op, in
           q1 *= f;
           q2 *= f;
           q3 *= f;
-          sum = fmaf(q0, q0, fmaf(q1, q1, fmaf(q2, q2, fmaf(q3, q3, sum))));
+          sum += f2d(fmaf(q0, q0, fmaf(q1, q1, fmaf(q2, q2, q3 * q3))));
           rp += plane;
           continue;
         }
@@ -406,7 +406,7 @@ __device__ __forceinline__ void cheb_pass(const ChebSys &S, const ChebOp &op, in
     if (CHECK) {
       double v[NR];
 #pragma unroll
-      for (int s = 0; s < NR; ++s) v[s] = rhs == s ? (double)sum : 0.0;
+      for (int s = 0; s < NR; ++s) v[s] = rhs == s ? sum : 0.0;
       block_sum<NR, kCGWarps, kChebThreads>(v, sred);
 #pragma unroll
       for (int s = 0; s < NR; ++s)
@@ -424,23 +424,22 @@ __device__ __forceinline__ void cheb_put(float *p, int k, int nz, float v) {
 
 // ---------------------------------------------------------------- residual
 // r = b - A (h + l) on the free DOFs in double-float arithmetic (l may be NULL), -0.0f on the pinned ones, and
-// the chunk partials of |r|^2 times scale^2 per right-hand side; b times `down` where that is set.  Every value
-// enters renormalised (h + l = hi + lo exactly, |lo| <= 2^-24 |hi|).  In units of 2^-48 of the sum of the terms'
+// the chunk partials of |r|^2 per right-hand side, of the unrounded r in FP64 (the stopping test is on this norm);
+// b times `down` where that is set.  Every value enters renormalised (h + l = hi + lo exactly, |lo| <= 2^-24 |hi|).  In units of 2^-48 of the sum of the terms'
 // magnitudes: the z and y sums of a term are within 8 (df_add: 3 per sum, twice, and 2 for the dropped
 // renormalisation), its product within 13 (df::fma), and the 4 + 4 accumulations and two sums of planes
 // within 3 each: 57, inside the 94 that the bound of df_error_bound allows.
 template <int NR>
 __device__ __forceinline__ void cheb_residual(const ChebSys &S, const ChebOp &op, int l, const double *down,
-                                              const float *h, const float *lo, float *r,
-                                              const float (&scale)[NR], double *half,
+                                              const float *h, const float *lo, float *r, double *half,
                                               double (*sred)[kCGWarps]) {
   const int nyz = S.ny * S.nz, nz = S.nz, P = S.pitch, q = NR * S.ny * P;
   for (int chunk = l; chunk < S.rchunks; chunk += S.ncta) {
     const int tile = chunk / S.rranges, x0 = (chunk - tile * S.rranges) * S.rlx, x1 = min(S.nx, x0 + S.rlx);
     const int f = tile * kChebThreads + threadIdx.x;
-    float nrm[NR];
+    double nrm[NR];
 #pragma unroll
-    for (int s = 0; s < NR; ++s) nrm[s] = 0.0f;
+    for (int s = 0; s < NR; ++s) nrm[s] = 0.0;
     if (f < nyz) {
       const int j = f / nz, k = f - j * nz;
       const int om = j == 0 ? (S.ny - 1) * P : -P, od = j == S.ny - 1 ? -(S.ny - 1) * P : P;
@@ -449,7 +448,7 @@ __device__ __forceinline__ void cheb_residual(const ChebSys &S, const ChebOp &op
         df::DF acc, sp;
         const int at = (s * S.ny + j) * P + k;
         const float *hs = h + at, *ls = lo ? lo + at : nullptr;
-        float sum = 0.0f;
+        double sum = 0.0;
 #pragma unroll 1
         for (int i = x0 - 1; i <= x1; ++i) {
           const int64_t p = (int64_t)(i < 0 ? S.nx - 1 : i >= S.nx ? 0 : i) * q;
@@ -471,10 +470,9 @@ __device__ __forceinline__ void cheb_residual(const ChebSys &S, const ChebOp &op
             float bh, bl;
             d2ff(down ? S.b[dof * NR + s] * down[s] : S.b[dof * NR + s], bh, bl);
             const df::DF d = df_add(df::DF(bh, bl), df::DF(-y.hi, -y.lo));
-            const float rv = pin ? -0.0f : (d.hi + d.lo) + 0.0f;
-            cheb_put(r + (int64_t)(i - 1) * q + at, k, nz, rv);
-            const float sv = rv * scale[s];
-            sum = fmaf(sv, sv, sum);
+            cheb_put(r + (int64_t)(i - 1) * q + at, k, nz, pin ? -0.0f : (d.hi + d.lo) + 0.0f);
+            const double t = pin ? 0.0 : f2d(d.hi) + f2d(d.lo);
+            sum = ::fma(t, t, sum);
           }
           acc = df_add(cc, sp);
           const float hi = __fadd_rn(acc.hi, acc.lo);
@@ -487,7 +485,7 @@ __device__ __forceinline__ void cheb_residual(const ChebSys &S, const ChebOp &op
     }
     double v[NR];
 #pragma unroll
-    for (int s = 0; s < NR; ++s) v[s] = (double)nrm[s];
+    for (int s = 0; s < NR; ++s) v[s] = nrm[s];
     block_sum<NR, kCGWarps, kChebThreads>(v, sred);
 #pragma unroll
     for (int s = 0; s < NR; ++s)
@@ -498,8 +496,7 @@ __device__ __forceinline__ void cheb_residual(const ChebSys &S, const ChebOp &op
 // The same in FP64 arithmetic.
 template <int NR>
 __device__ __noinline__ void cheb_residual64(const ChebSys &S, const ChebOp &op, int l, const double *down,
-                                             const float *h, const float *lo, float *r,
-                                              const float (&scale)[NR], double *half,
+                                             const float *h, const float *lo, float *r, double *half,
                                              double (*sred)[kCGWarps]) {
   const int nyz = S.ny * S.nz, nz = S.nz, P = S.pitch, q = NR * S.ny * P;
   for (int chunk = l; chunk < S.rchunks; chunk += S.ncta) {
@@ -532,7 +529,7 @@ __device__ __noinline__ void cheb_residual64(const ChebSys &S, const ChebOp &op,
           cheb_put(r + (int64_t)i * q + (s * S.ny + j) * P + k, k, nz, pin ? -0.0f : (float)t + 0.0f);
 #pragma unroll
           for (int e = 0; e < NR; ++e)
-            if (e == s) nrm[e] = ::fma(t * (double)scale[e], t * (double)scale[e], nrm[e]);
+            if (e == s) nrm[e] = ::fma(t, t, nrm[e]);
         }
       }
     }
@@ -650,7 +647,7 @@ __device__ __forceinline__ bool cheb_solve(const ChebSys &S, const ChebOp &op, i
           st.scaled = 1;
           bb = ldexp(bb, -2 * e);
         }
-        if (st.fit) st.exp2[s] = ilogb(bb) / 2;  // |r|^2 is summed in FP32 over r / 2^exp2, 2^exp2 near ||b||
+        if (st.fit) st.exp2[s] = ilogb(bb) / 2;  // the check squares in FP32 over r / 2^exp2, 2^exp2 near ||b||
         st.scale[s] = (float)ldexp(1.0, -st.exp2[s]);
       }
       st.bn[s] = st.res[s] = sqrt(bb);
@@ -683,15 +680,15 @@ __device__ __forceinline__ bool cheb_solve(const ChebSys &S, const ChebOp &op, i
       if (!first || use_init) {
         // ---- the residual of x = h + lo
         double *half = S.part + (size_t)par * S.half;
-        if (op.df) cheb_residual<NR>(S, op, l, down, h, lo, r, scale, half, sred);
-        else cheb_residual64<NR>(S, op, l, down, h, lo, r, scale, half, sred);
+        if (op.df) cheb_residual<NR>(S, op, l, down, h, lo, r, half, sred);
+        else cheb_residual64<NR>(S, op, l, down, h, lo, r, half, sred);
         double t[NR];
         if (!cheb_totals<NR>(S, tns, S.rchunks, par, t, sred)) { status = CPM_BARRIER_TIMEOUT; break; }
         if (!first) ++updates;
         if (threadIdx.x == 0) {
           st.finite = 1;
           for (int s = 0; s < NR; ++s) {
-            st.res[s] = ldexp(sqrt(t[s]), st.exp2[s]);
+            st.res[s] = sqrt(t[s]);
             if (!((st.pending >> s) & 1)) continue;
             if (!isfinite(st.res[s])) st.finite = 0;
             // a double-float residual decides outside its error bound only; a warm start takes at least

@@ -102,3 +102,23 @@ def test_fp64_residuals_decide_where_they_are_asked_for(name, nrhs):
         tol = 64 * 2.0 ** -53 * np.abs(op.coef_host).sum() * np.linalg.norm(xx[:, r])
         assert res <= TOL * np.linalg.norm(bb[:, r])
         assert abs(inf["resid"][r] - res) <= tol, (inf["resid"][r], res, tol)
+
+
+def test_residual_norm_that_decides_is_summed_in_fp64():
+    """b = 1 without pinned DOFs: every node holds the same residual, and a loose tolerance with a warm start of
+    1.2e6 half tolerances ends on a double-float residual after one cycle.  Its norm is that of x to the double-float
+    bound, 128 * 2^-48 sum|c| max|x| per node, and 512 roundings of FP64 sums (256 equal squares per thread in FP32
+    would be off by 1e-7)."""
+    from fractions import Fraction
+    from cupymag_gb300.utils.stencil_operator import StencilOperator
+    coef = _case((4, 4, 4), 0)[1]["A1"].coef_host
+    op = StencilOperator(256, 280, 280, coef)
+    tol = 1e-2
+    b = np.ones(op.n)
+    x, inf = _solve(op, b, np.full(op.n, 1.0 + 1.2e6 * 0.5 * tol), tol=tol)
+    assert inf["status"] == 0 and inf["outer"] == inf["df_updates"] == 1, inf
+    assert np.all(x == x[0])
+    r = abs(float(1 - sum(Fraction(float(c)) for c in coef) * Fraction(float(x[0]))))
+    assert 0.1 * tol < r <= tol
+    err = 128 * 2.0 ** -48 * np.abs(coef).sum() * abs(x[0]) / r + 512 * 2.0 ** -53
+    assert abs(inf["resid"][0] / (r * np.sqrt(op.n)) - 1) <= err, (inf["resid"][0], r * np.sqrt(op.n), err)
