@@ -122,3 +122,67 @@ def test_residual_norm_that_decides_is_summed_in_fp64():
     assert 0.1 * tol < r <= tol
     err = 128 * 2.0 ** -48 * np.abs(coef).sum() * abs(x[0]) / r + 512 * 2.0 ** -53
     assert abs(inf["resid"][0] / (r * np.sqrt(op.n)) - 1) <= err, (inf["resid"][0], r * np.sqrt(op.n), err)
+
+
+def _residuals(A, b, x):
+    n = b.shape[0]
+    bb, xx = b.reshape(n, -1), x.reshape(n, -1)
+    return [np.linalg.norm(bb[:, r] - A @ xx[:, r]) / np.linalg.norm(bb[:, r]) for r in range(bb.shape[1])]
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -200, 2.0 ** 300])
+@pytest.mark.parametrize("df", [True, False])
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_warm_start_far_from_the_solution_takes_several_cycles(nrhs, df, scale):
+    """Three and more cycles (corrections beyond the pair of a cold start), in both residual forms and with
+    right-hand sides that are scaled down and up; pinned DOFs are exact."""
+    from cupymag_gb300.solvers.linear_solvers import CGSolver
+    S, so, csr = _case((9, 12, 7), 2)
+    A, op = csr["A2"], so["A2"]
+    rng = np.random.default_rng(11)
+    b = rng.normal(size=(op.n, 3) if nrhs == 3 else op.n)
+    x0 = 1e4 * rng.normal(size=b.shape)
+    solver = CGSolver()
+    solver.df_residual = df
+    x, inf = _solve(op, scale * b, scale * x0, solver=solver)
+    assert inf["status"] == 0 and inf["outer"] >= 2, inf
+    assert max(_residuals(A, b, x / scale)) <= TOL
+    assert np.array_equal(x[S.DefDOF], scale * b[S.DefDOF])
+    y, _ = _solve(op, b, x0, solver=solver)
+    assert np.array_equal(scale * y, x)
+
+
+@pytest.mark.parametrize("nz", [5, 8])
+@pytest.mark.parametrize("ratio", [0.02, 0.0158])
+def test_wide_spectrum(ratio, nz):
+    """Condition numbers of 50 and 63 (a cycle's FP32 rounding leaves more for the next): the stopping test holds,
+    cold and warm, with either residual."""
+    from cupymag_gb300.solvers.linear_solvers import CGSolver
+    from cupymag_gb300.utils.stencil_operator import StencilOperator
+    t = (1 - ratio ** (1 / 3)) / 4   # symbol of the tensor product: (1 - 2 t + 2 t cos)^3, between 1 and `ratio`
+    one = np.array([t, 1 - 2 * t, t])
+    op = StencilOperator(11, 6, nz, np.einsum("a,b,c->abc", one, one, one).reshape(27))
+    rng = np.random.default_rng(1)
+    b = rng.normal(size=op.n)
+    for df in (True, False):
+        solver = CGSolver()
+        solver.df_residual = df
+        for x0 in (None, rng.normal(size=op.n)):
+            x, inf = _solve(op, b, x0, tol=1e-9, solver=solver)
+            r = b - op.spmv(torch.as_tensor(x, device="cuda")).cpu().numpy()
+            assert inf["status"] == 0 and np.linalg.norm(r) <= 1e-9 * np.linalg.norm(b), inf
+
+
+@pytest.mark.parametrize("name,steps", [("A1", 40), ("A2", 60)])
+def test_the_default_form_runs_the_schedule(name, steps):
+    """Cold solves to 1e-10 take the iteration's own step count (one less or more by the sizes of the two cycles) on
+    every grid, with double-float residuals, where CG's count depends on the grid and the right-hand side."""
+    for dims in ((8, 9, 10), (21, 5, 33), (30, 28, 26)):
+        op = _case(dims, 2)[1][name]
+        for nrhs in (1, 3):
+            b = np.random.default_rng(dims[2]).normal(size=(op.n, 3) if nrhs == 3 else op.n)
+            _, inf = _solve(op, b)
+            _, cg = _solve(op, b, form=1)
+            assert inf["status"] == 0 and abs(inf["iters"][0] - steps) <= 1, inf
+            assert inf["iters"][:nrhs] == inf["iters"][:1] * nrhs and inf["outer"] == inf["df_updates"] == 1, inf
+            assert cg["iters"][0] < steps - 2, cg
