@@ -1182,7 +1182,7 @@ extern "C" int cpm_cg_solve_stencil_fft(const cpm_stencil *S, const cpm_fft_prec
   a.cb = o->carry_b;
   a.ct = o->carry_t;
   a.carry_valid = o->carry_valid;
-  if (nc == 3) a.even = even3_coefs(S->coef, a.e64);  // the pair-summed FP64 residual
+  if (nc == 3) a.even = even3_coefs(S->coef, a.e64, 1e-12);  // the pair-summed FP64 residual
   a.lx = nc == 1 && even8_coefs(S->coef, a.c8) ? even8_planes(S->nx, (int64_t)S->ny * S->nz, sm_count()) : 0;
   const bool slab = P->layout == CPM_FFT_LAYOUT_SLAB;
   const void *fn = slab ? (nc == 3 ? (const void *)cg_stencil_fft_kernel<3, CPM_FFT_LAYOUT_SLAB>

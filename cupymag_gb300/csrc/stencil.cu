@@ -1119,7 +1119,7 @@ static int launch_stencil_cg(const cpm_stencil *s, const double *b, double *x, c
       }
     }
   }
-  if (fp64 && NC == 3) a.even = even3_coefs(s->coef, a.e64);
+  if (fp64 && NC == 3) a.even = even3_coefs(s->coef, a.e64, kEvenRounding);
   if constexpr (NC == 1) {
     if (!fp64) {
       a.quads = quads_ok(s) && ((uintptr_t)x & 15) == 0 ? 1 : 0;

@@ -173,9 +173,12 @@ __device__ __forceinline__ void elastic_rows(const Geo &S, const T *c, const XS 
       }
 }
 
-// Coefficients of the pair form of an elastic stencil even in the offset (c(-d) = c(d) to 1e-12 of each block's
+// Coefficients of the pair form of an elastic stencil even in the offset (c(-d) = c(d) to `rel` of each block's
 // largest): the even part (c(d) + c(26 - d)) / 2 per block for d < 13, then c(13).  1 if it applies.
-inline int even3_coefs(const double *coef, double *e64) {
+// rel: kEvenRounding where the product has to be the operator's to FP64 rounding (the FP64 CG), 1e-12 in the FFT
+// solve's residuals.
+constexpr double kEvenRounding = 1e-15;
+inline int even3_coefs(const double *coef, double *e64, double rel) {
   int even = 1;
   for (int blk = 0; blk < 9; ++blk) {
     const double *c = coef + 27 * blk;
@@ -183,7 +186,7 @@ inline int even3_coefs(const double *coef, double *e64) {
     for (int d = 0; d < 27; ++d) big = c[d] > big ? c[d] : -c[d] > big ? -c[d] : big;
     for (int d = 0; d < 13; ++d) {
       const double o = c[d] - c[26 - d];
-      if (o > 1e-12 * big || -o > 1e-12 * big) even = 0;
+      if (o > rel * big || -o > rel * big) even = 0;
       e64[blk * 14 + d] = 0.5 * (c[d] + c[26 - d]);
     }
     e64[blk * 14 + 13] = c[13];
@@ -220,7 +223,7 @@ __device__ __forceinline__ void even3_rows(const Geo &S, const double *e64, cons
 
 // ---------------------------------------------------------------- FP64 products of even scalar stencils
 // The 8 coefficients c[4 |dx| + 2 |dy| + |dz|] of a scalar stencil even along every axis; false unless that is all
-// of it, to 1e-15 of the largest coefficient.
+// of it, to kEvenRounding of the largest coefficient.
 inline bool even8_coefs(const double *coef, double *c8) {
   double big = 0.0;
   for (int e = 0; e < 8; ++e) c8[e] = 0.0;
@@ -231,7 +234,7 @@ inline bool even8_coefs(const double *coef, double *c8) {
   }
   for (int d = 0; d < 27; ++d) {
     const double o = coef[d] - c8[4 * (d / 9 != 1) + 2 * ((d / 3) % 3 != 1) + (d % 3 != 1)];
-    if (!(o <= 1e-15 * big && -o <= 1e-15 * big)) return false;
+    if (!(o <= kEvenRounding * big && -o <= kEvenRounding * big)) return false;
   }
   return true;
 }

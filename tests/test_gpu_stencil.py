@@ -329,3 +329,45 @@ def test_product_of_three_vectors_finds_the_flags_beyond_2_32_values():
     finally:
         del x, y
         torch.cuda.empty_cache()
+
+
+def test_fp64_cg_solves_the_elastic_operator_as_given():
+    """An elastic stencil that is even only to 4e-13 (blocks (p, q) and (q, p) carry opposite odd parts, so the operator
+    stays symmetric): FP64 CG solves that operator.  The residual of its solution is at the rounding of FP64 CG; the
+    symmetrised operator's solution leaves the odd part's, hundreds of times as much."""
+    from cupymag_gb300.solvers.linear_solvers import CGSolver, decode_info, new_info
+    from cupymag_gb300.utils.stencil_operator import StencilOperator
+    rng = np.random.default_rng(12)
+    c = np.zeros((3, 3, 27))
+    for p in range(3):
+        for q in range(p, 3):
+            v = rng.uniform(-0.02, 0.02, size=27)
+            c[p, q] = c[q, p] = v + v[::-1]
+        c[p, p, 13] = 3.0
+    c[0, 1, 13] = c[1, 0, 13] = 1.0
+    odd = 4e-13 * np.sign(rng.normal(size=27))
+    odd = (odd - odd[::-1]) / 2
+    c[0, 1] += odd
+    c[1, 0] -= odd
+    dims = (7, 6, 5)
+    op = StencilOperator(*dims, c.reshape(-1))
+    b = rng.normal(size=3 * op.n)
+    bd = torch.as_tensor(b, device="cuda")
+    x, info = torch.zeros_like(bd), new_info(1)
+    CGSolver().launch(op, bd, x, info[0], tol=1e-15, maxiter=60, precision="DP")
+    assert decode_info(info[0].cpu().numpy())["status"] in (0, 1)
+    u = x.cpu().numpy().reshape(3, *dims)
+    off = [(i, j, k) for i in (-1, 0, 1) for j in (-1, 0, 1) for k in (-1, 0, 1)]
+    roll = lambda v, d: np.roll(v, [-o for o in off[d]], (0, 1, 2))  # noqa: E731
+    # even and odd parts apart, so that the odd part's product is exact to its own rounding
+    even = c.copy()
+    even[0, 1], even[1, 0] = c[0, 1] - odd, c[1, 0] + odd
+    y = np.stack([sum(even[p, q, d] * roll(u[q], d) for q in range(3) for d in range(27)) for p in range(3)])
+    z = np.zeros_like(y)
+    z[0] = sum(odd[d] * roll(u[1], d) for d in range(27))
+    z[1] = -sum(odd[d] * roll(u[0], d) for d in range(27))
+    r = np.linalg.norm(b - (y + z).reshape(-1))
+    assert np.linalg.norm(z) >= 1e-13 * np.linalg.norm(b)
+    # 60 iterations' updates and a product of 81 terms, each within 2^-53 of sum|c| |x| (typically their root)
+    assert r <= 30 * 2.0 ** -53 * np.abs(c).sum(axis=(1, 2)).max() * np.linalg.norm(u), (r, np.linalg.norm(z))
+    assert r <= 0.25 * np.linalg.norm(z), (r, np.linalg.norm(z))
