@@ -652,11 +652,8 @@ __device__ __forceinline__ void true_residual64(const FftCGArgs &a, int64_t d0, 
         if (g >= nyz) continue;
         even8_march<1>(a.c8, a.x, a.S.nx, a.S.ny, a.S.nz, g, xa, min(a.S.nx, xa + a.lx), [&](int i, double y) {
           const int64_t o = (int64_t)i * nyz + g;
-          if (a.S.flags && a.S.flags[o]) {
-            double u[1];
-            apply<double, 1, 1>(a.S, a.x, (int)o, u);
-            y = u[0];
-          }
+          const int fl = a.S.flags ? a.S.flags[o] : 0;
+          if (fl) y = flagged_row<1>(a.S, a.x, (int)o, 0, fl);
           const double bi = a.b[o], t = bi - y;
           a.r[o] = (float)t;
           if (!SUMS) a.d[o] = 0.0f;

@@ -831,9 +831,13 @@ __global__ void __launch_bounds__(256) stencil_apply_kernel(const __grid_constan
   }
 }
 
-// The same for scalar stencils even along every axis, marching along x (even8_march); rows with flags take the per-DOF
-// product.  Measured on GB300, us per product with 1 and 3 vectors, the forms above / this: 128^3 118, 350 / 72, 213;
-// 64^3 18.7, 51.8 / 14.9, 31.5; 36^3 10.3, 27.0 / 6.4, 10.5; 28x31x26 4.4, 8.3 / 4.8, 6.5.
+// The same for scalar stencils even along every axis, marching along x (even8_march); rows with flags by flagged_row.
+// Measured on GB300, us per product, per DOF / this, with one vector: without flags 30^3 3.9 / 4.3, 45x41x49
+// 8.0 / 8.4, 5x64x512 12.1 / 13.2, 59^3 14.2 / 11.8, 128^3 115 / 72; with a defect of a sixth of the edge 45x41x49
+// 10.1 / 11.0, 64^3 18.5 / 20.3, 85^3 37.4 / 43.0, 96^3 52.8 / 46.8, 128^3 121 / 84.  With three: without flags 20^3
+// 8.0 / 4.2, 30^3 8.1 / 8.4, 512x8x8 8.1 / 10.7, 34^3 14.4 / 10.7, 128^3 337 / 213; with the defect 20^3 11.3 / 7.5,
+// 32^3 11.1 / 10.8, 48^3 24.6 / 26.7, 64^3 50.9 / 41.6, 128^3 353 / 212.  (Quads of scalar even stencils, the form
+// for nz % 4 == 0 before, are slower than both: 20^3 with flags 21.)
 template <int NR>
 __global__ void __launch_bounds__(128) stencil_march_kernel(const __grid_constant__ StencilOp S,
                                                             const __grid_constant__ Even8 e, const double *x,
@@ -846,15 +850,18 @@ __global__ void __launch_bounds__(128) stencil_march_kernel(const __grid_constan
   const uint8_t *flags = S.flags;
   even8_march<NR>(e.c, x, S.nx, S.ny, S.nz, g, x0, x1, [&](int i, double v) {
     const int dof = i * nyz + f;  // below 2^31; value indices need 64 bits (up to 3 x 2^31)
-    if (flags && flags[dof]) {
-      double t[NR];
-      apply<double, 1, NR>(S, x, dof, t);
-#pragma unroll
-      for (int r = 0; r < NR; ++r)
-        if (g - f * NR == r) v = t[r];
-    }
+    const int fl = flags ? flags[dof] : 0;
+    if (fl) v = flagged_row<NR>(S, x, dof, g - f * NR, fl);
     y[(int64_t)i * values + g] = alpha * v;
   });
+}
+
+// Whether the march is the faster form (the figures above).  One vector: too few columns to fill the GPU below the
+// line, and a march's flagged rows are a serial chain that only larger grids hide.  Three vectors: only where all
+// nodes fit one block per SM is the product per DOF ahead, and not by rows with flags.
+static bool march_pays(const StencilOp &S, int nvec) {
+  if (nvec == 1) return S.n >= (S.flags ? 700000 : 170000);
+  return S.flags || S.n < 27000 || S.n > sm_count() * 256;
 }
 
 // ---------------------------------------------------------------- y = A x (FP32, the refinement form's product)
@@ -1233,7 +1240,8 @@ extern "C" int cpm_stencil_apply(const cpm_stencil *S, const double *x, double *
   }
   const StencilOp op = to_op(S);
   Even8 e;
-  if (S->ncomp == 1 && even8_coefs(S->coef, e.c)) {
+  const bool even = S->ncomp == 1 && even8_coefs(S->coef, e.c);
+  if (even && march_pays(op, nvec)) {
     const int64_t values = (int64_t)S->ny * S->nz * nvec;
     const int lx = even8_planes(S->nx, values, sm_count());
     const dim3 grid((unsigned)((values + 127) / 128), (unsigned)((S->nx + lx - 1) / lx));
@@ -1247,7 +1255,7 @@ extern "C" int cpm_stencil_apply(const cpm_stencil *S, const double *x, double *
   const int64_t cap = (int64_t)sm_count() * 8;
   if (g > cap) g = cap;
   cudaStream_t st = (cudaStream_t)stream;
-  if (quads_ok(S) && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
+  if (!even && quads_ok(S) && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
     const int64_t gq = std::max<int64_t>(1, std::min<int64_t>(g, (op.n / 4 + 255) / 256));
     if (S->ncomp == 3)
       stencil_apply4_kernel<3, 1><<<(int)gq, 256, 0, st>>>(op, x, y, alpha);

@@ -371,3 +371,34 @@ def test_fp64_cg_solves_the_elastic_operator_as_given():
     # 60 iterations' updates and a product of 81 terms, each within 2^-53 of sum|c| |x| (typically their root)
     assert r <= 30 * 2.0 ** -53 * np.abs(c).sum(axis=(1, 2)).max() * np.linalg.norm(u), (r, np.linalg.norm(z))
     assert r <= 0.25 * np.linalg.norm(z), (r, np.linalg.norm(z))
+
+
+@pytest.mark.parametrize("nvec", [1, 3])
+@pytest.mark.parametrize("dims", [(3, 3, 3), (5, 4, 7), (16, 9, 12), (30, 30, 30), (31, 33, 34), (88, 90, 89)])
+def test_products_of_even_scalar_stencils_on_both_sides_of_the_lines(dims, nvec):
+    """The mass-like product with unit, empty and excluded rows and columns, and without flags, on grids that take the
+    march and on grids that take the product per node: each value within 64 roundings of the sum of its terms."""
+    from cupymag_gb300.utils.stencil_operator import COL_EXCLUDED, ROW_IDENTITY, ROW_ZERO, StencilOperator
+    rng = np.random.default_rng(sum(dims) + nvec)
+    c8 = rng.uniform(-1.0, 1.0, size=8)
+    coef = np.array([c8[4 * (d // 9 != 1) + 2 * (d // 3 % 3 != 1) + (d % 3 != 1)] for d in range(27)])
+    n = dims[0] * dims[1] * dims[2]
+    x = rng.normal(size=(n, 3) if nvec == 3 else n)
+    for flagged in (False, True):
+        f = np.zeros(n, dtype=np.uint8)
+        if flagged:
+            q = rng.permutation(n)[:12]
+            f[q[:4]], f[q[4:8]], f[q[8:]] = ROW_IDENTITY | COL_EXCLUDED, ROW_ZERO | COL_EXCLUDED, COL_EXCLUDED
+        op = StencilOperator(*dims, coef, f if flagged else None)
+        y = op.spmv(torch.as_tensor(x, device="cuda")).cpu().numpy().reshape(n, -1)
+        v = np.where(((f & COL_EXCLUDED) != 0)[:, None], 0.0, x.reshape(n, -1)).reshape(*dims, nvec)
+        ref, mag = np.zeros_like(v), np.zeros_like(v)
+        for d in range(27):
+            t = coef[d] * np.roll(v, (1 - d // 9, 1 - d // 3 % 3, 1 - d % 3), (0, 1, 2))
+            ref += t
+            mag += np.abs(t)
+        ref, mag = ref.reshape(n, -1), mag.reshape(n, -1)
+        unit, empty = (f & ROW_IDENTITY) != 0, (f & ROW_ZERO) != 0
+        ref[unit], mag[unit] = x.reshape(n, -1)[unit], 0.0
+        ref[empty], mag[empty] = 0.0, 0.0
+        assert np.all(np.abs(y - ref) <= 64 * 2.0 ** -53 * mag), (dims, nvec, flagged)
