@@ -644,8 +644,7 @@ __device__ __forceinline__ void true_residual64(const FftCGArgs &a, int64_t d0, 
   for (int j = 0; j < NV; ++j) v[j] = 0.0;
   if constexpr (NC == 1) {
     if (a.lx > 0 && !x0) {
-      // marches over columns of the grid, dealt to the CTAs in turn (the next phase reads r past a barrier):
-      // the cold 192x192x180 demag solve 1865 -> 1618 us on GB300
+      // marches over columns of the grid, dealt to the CTAs in turn (the next phase reads r past a barrier)
       const int nyz = a.S.ny * a.S.nz, tiles = (nyz + NT - 1) / NT, ranges = (a.S.nx + a.lx - 1) / a.lx;
       for (int t = blockIdx.x; t < tiles * ranges; t += gridDim.x) {
         const int q = t / ranges, g = q * NT + threadIdx.x, xa = (t - q * ranges) * a.lx;
@@ -980,6 +979,29 @@ static size_t fft_cg_layout(int64_t n, int nc, char *base, Workspace *w, float2 
   return off;
 }
 
+// The marching residual of scalar stencils takes grids of this many nodes; smaller ones lack columns.  Measured on
+// GB300, us per cold demag solve, per node / march: 32^3 83 / 92, 56^3 129 / 133, 59^3 179 / 179, 64^3 127 / 125,
+// 80^3 199 / 191, 96^3 240 / 208, 110x112x105 369 / 327, 300x300x10 306 / 275, 10x300x300 350 / 348, 128^3 436 / 366.
+constexpr int64_t kMarchResidual = 200000;
+
+// Planes per march: `tiles` columns of a block's threads are dealt to G blocks, which run them one after the other,
+// and a march's two rim planes cost about 1.2 output planes.  (16 planes for every grid left the last round of blocks
+// nearly empty: 108^3 348 us where this takes 268.)
+static int residual_planes(int nx, int64_t tiles, int64_t G) {
+  int lx = nx;
+  double best = 1e300;
+  for (int nr = 1; nr <= nx; ++nr) {
+    const int l = (nx + nr - 1) / nr;
+    const int64_t rounds = (tiles * ((nx + l - 1) / l) + G - 1) / G;
+    const double cost = (double)rounds * (l + 1.2);
+    if (cost < best) {
+      best = cost;
+      lx = l;
+    }
+  }
+  return lx;
+}
+
 }  // namespace cpm
 
 extern "C" int64_t cpm_fft_precond_bytes(int32_t nx, int32_t ny, int32_t nz, int32_t ncomp) {
@@ -1180,7 +1202,6 @@ extern "C" int cpm_cg_solve_stencil_fft(const cpm_stencil *S, const cpm_fft_prec
   a.ct = o->carry_t;
   a.carry_valid = o->carry_valid;
   if (nc == 3) a.even = even3_coefs(S->coef, a.e64, 1e-12);  // the pair-summed FP64 residual
-  a.lx = nc == 1 && even8_coefs(S->coef, a.c8) ? even8_planes(S->nx, (int64_t)S->ny * S->nz, sm_count()) : 0;
   const bool slab = P->layout == CPM_FFT_LAYOUT_SLAB;
   const void *fn = slab ? (nc == 3 ? (const void *)cg_stencil_fft_kernel<3, CPM_FFT_LAYOUT_SLAB>
                                    : (const void *)cg_stencil_fft_kernel<1, CPM_FFT_LAYOUT_SLAB>)
@@ -1204,6 +1225,8 @@ extern "C" int cpm_cg_solve_stencil_fft(const cpm_stencil *S, const cpm_fft_prec
   G = std::max<int64_t>(1, (n + per - 1) / per);
   a.dofs_per_cta = per;
   a.F = grid_of(P, C, G);
+  if (nc == 1 && n >= kMarchResidual && even8_coefs(S->coef, a.c8))
+    a.lx = residual_planes(S->nx, ((int64_t)S->ny * S->nz + threads - 1) / threads, G);
   CPM_TRY(cudaMemsetAsync(w.bar, 0, sizeof(GridBarrier), (cudaStream_t)stream));
   CPM_TRY(cudaMemsetAsync(info, 0, sizeof(cpm_cg_info), (cudaStream_t)stream));
   void *args[] = {&a};

@@ -274,3 +274,49 @@ def test_direct_solve_residual_carry(layout):
         alias = types.SimpleNamespace(b=x, t=carry.t, valid=carry.valid)
         with pytest.raises(RuntimeError, match="alias"):
             solve(b0, x, True, carry=alias)
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("method", METHODS)
+@pytest.mark.parametrize("dims", [(64, 63, 50), (9, 150, 160), (300, 27, 25)])
+def test_marching_residual_keeps_the_fp64_stopping_test(dims, method, layout):
+    """Demag solves on grids that take the marching FP64 residual (200 k nodes and more; long, flat and ragged marches):
+    ||b - A x|| <= tol ||b|| on the host, the residual that the solve reports is that of x to the rounding of the
+    product (64 * 2^-53 sum|c| ||x||), cold and warm with a carry, and a zero right-hand side returns zeros."""
+    from cupymag_gb300 import _native as N
+    from cupymag_gb300.solvers.linear_solvers import CGSolver, ResidualCarry, decode_info, new_info
+    from cupymag_gb300.utils.stencil_operator import COL_EXCLUDED, ROW_IDENTITY, StencilOperator
+    S, _ = _sim(Nx=6, Ny=6, Nz=6, Ndx=0, Ndy=0, Ndz=0)
+    n = dims[0] * dims[1] * dims[2]
+    f = np.zeros(n, dtype=np.uint8)
+    f[0] = ROW_IDENTITY | COL_EXCLUDED
+    coef = S.stencil_operators()["A_demag"].coef_host
+    op = StencilOperator(*dims, coef, f)
+    rng = np.random.default_rng(dims[0])
+    solver = CGSolver()
+    solver.fft_layout = _layout(layout)
+    if op.fft_plan(solver.fft_layout) is None:
+        pytest.skip("no plan of this layout for the grid")
+    form = N.CG_FORM_DEFAULT if method == "direct" else N.CG_FORM_FFT_PCG
+    carry, info = ResidualCarry(n), new_info(1)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    for warm in (False, True):
+        b = rng.normal(size=n)
+        b[0] = 0.0
+        solver.launch(op, torch.as_tensor(b, device="cuda"), x, info[0], tol=1e-10, maxiter=2000, precision="IR",
+                      use_init=warm, precond="fft", form=form, carry=carry)
+        inf = decode_info(info[0].cpu().numpy())
+        assert inf["status"] == 0, inf
+        u = x.cpu().numpy().reshape(dims).copy()
+        anchor, u[0, 0, 0] = u[0, 0, 0], 0.0   # a unit row; its column is left out of the others
+        y = np.zeros(dims)
+        for d in range(27):
+            y += coef[d] * np.roll(u, (1 - d // 9, 1 - d // 3 % 3, 1 - d % 3), (0, 1, 2))
+        r = b - y.reshape(-1)
+        r[0] = -anchor
+        assert method == "pcg" or anchor == 0.0
+        res = np.linalg.norm(r)
+        assert res <= 1e-10 * np.linalg.norm(b) * 1.001, inf
+        assert abs(res - inf["resid"][0]) <= 64 * 2.0 ** -53 * np.abs(coef).sum() * np.linalg.norm(u), (inf, res)
+    solver.launch(op, torch.zeros_like(x), x, info[0], tol=1e-10, maxiter=2000, precision="IR", precond="fft", form=form)
+    assert decode_info(info[0].cpu().numpy())["status"] == 0 and not x.any()
