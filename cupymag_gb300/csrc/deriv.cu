@@ -272,6 +272,7 @@ struct MirrorArgs {
 };
 
 constexpr int kTileThreads = 256;
+constexpr double kPipeUs = 0.0096;  // of an SM's FP64 pipe per warp instruction: 16 cycles, at 80 to 90 % of them busy
 constexpr int kTileRim = 350;  // nodes of a tile with its rim at most
 
 // Parts of a field's derivatives from its values t (shared memory, z-lines of w): Fx from the x difference of
@@ -438,8 +439,9 @@ __global__ void __launch_bounds__(kTileThreads, 2) mirror_kernel(const __grid_co
 // Tile and planes per block.  Tile: the fewest FP64 warp instructions (`out` per output, `rim` per node of the tile
 // and its rim).  Planes: the blocks of one SM run one after the other on its FP64 pipe, and the two rim planes of a
 // range cost about 0.8 of an output plane.
-static bool mirror_shape(MirrorArgs &m, double out, double rim) {
-  double best = 1e300;
+// Returns the march's time by that model in us (see march_pays), negative where the grid has no tile.
+static double mirror_shape(MirrorArgs &m, double out, double rim) {
+  double best = 1e300, plane = 0.0;
   for (int nt = 1; nt <= m.nz; ++nt) {
     const int z = (m.nz + nt - 1) / nt;
     if (z > 128) continue;
@@ -447,18 +449,20 @@ static bool mirror_shape(MirrorArgs &m, double out, double rim) {
     int t = std::min(std::min(kTileThreads / z, kTileRim / (z + 2) - 2), m.ny);
     if (t < 1) continue;
     t = (m.ny + (m.ny + t - 1) / t - 1) / ((m.ny + t - 1) / t);
-    const double cost = (double)((m.nz + z - 1) / z) * ((m.ny + t - 1) / t) *
-                        ((t * z + 31) / 32 * out + ((t + 2) * (z + 2) + 31) / 32 * rim);
+    const double block = (t * z + 31) / 32 * out + ((t + 2) * (z + 2) + 31) / 32 * rim;
+    const double cost = (double)((m.nz + z - 1) / z) * ((m.ny + t - 1) / t) * block;
     if (cost < best) {
       best = cost;
+      plane = block;
       m.tz = z;
       m.ty = t;
     }
   }
-  if (best >= 1e300) return false;
+  if (best >= 1e300) return -1.0;
   m.ntz = (m.nz + m.tz - 1) / m.tz;
   const int64_t tiles = (int64_t)m.ntz * ((m.ny + m.ty - 1) / m.ty);
   const int sms = sm_count();
+  double us = 0.0;
   best = 1e300;
   for (int nr = 1; nr <= m.nx && nr <= 65535; ++nr) {
     const int l = (m.nx + nr - 1) / nr;
@@ -467,9 +471,23 @@ static bool mirror_shape(MirrorArgs &m, double out, double rim) {
     if (cost < best) {
       best = cost;
       m.lx = l;
+      us = kPipeUs * 1.07 * per * (l + 0.8) * plane + 0.4 * (l + 2);
     }
   }
-  return tiles < (1ll << 31);
+  return tiles < (1ll << 31) ? us : -1.0;
+}
+
+// Whether a march of `us` (mirror_shape) and `start` us to begin with beats the pair kernel of `ops` FP64 operations
+// per node: both wait on the FP64 pipe, the pair kernel in whole rounds of one 256-node block per SM, the march in
+// blocks per SM times planes, plus 0.4 us a plane of latency.  Within 10 % of the times measured on GB300 on 70 grids
+// from 8^3 to 128^3, among them films and bars (3x200x140, 600x600x4, 512x8x8), and never the slower form by more
+// than 2 % there.  Us, pairs / march: F_el 25x27x29 25.2 / 27.9, 38^3 48.6 / 52.4, 40^3 48.6 / 33.2, 128^3 1248 / 653;
+// strain 53^3 70.6 / 75.2, 64^3 98.1 / 91.7, 64x512x5 70.7 / 73.4, 256x4x256 98.1 / 75.1; right-hand side 20^3
+// 7.7 / 7.2, 33x31x35 7.9 / 11.1, 128^3 325 / 143; Hd 53^3 22.2 / 23.9, 64^3 30.4 / 27.9, 128^3 222 / 156.
+static bool march_pays(double us, double start, int64_t n, double ops) {
+  const int64_t rounds = ((n + kDerivThreads - 1) / kDerivThreads + sm_count() - 1) / std::max(1, sm_count());
+  const double warps = (double)std::min<int64_t>(kDerivThreads / 32, (n + 31) / 32);
+  return us >= 0.0 && n >= kDerivThreads && us + start < kPipeUs * rounds * warps * ops + 1.0;
 }
 
 // The part of a 27-point stencil odd along `axis` and even along the other two, c[2 b + c] at the axis' +1
@@ -501,19 +519,14 @@ static double largest(const double *v, int count) {
   return big;
 }
 
-// The march needs enough columns: below `from` nodes the pair kernels (one thread per node) are faster.  Measured on
-// GB300, us pairs / march: F_el 28x31x26 25.4 / 27.9, 36^3 48.7 / 47.4; strain 36^3 29.7 / 33.2, 45x41x49
-// 43.4 / 38.9; Hd 36^3 10.1 / 11.6, 45x41x49 14.1 / 13.7; the right-hand side gains at every size (20^3 7.9 / 6.9).
-constexpr int64_t kMarchFel = 40000, kMarchDeriv = 80000;
-
-static bool mirror_deriv(const cpm_deriv_stencil *D, MirrorArgs &m, double out, double rim, int64_t from) {
-  if ((int64_t)D->nx * D->ny * D->nz < from) return false;
+static bool mirror_deriv(const cpm_deriv_stencil *D, MirrorArgs &m, double out, double rim, double start, double ops) {
   m = MirrorArgs{};
   m.nx = D->nx;
   m.ny = D->ny;
   m.nz = D->nz;
-  return mirror_part(D->fx, 0, largest(D->fx, 27), m.c.p) && mirror_part(D->fy, 1, largest(D->fy, 27), m.c.q) &&
-         mirror_part(D->fz, 2, largest(D->fz, 27), m.c.r) && mirror_shape(m, out, rim);
+  return march_pays(mirror_shape(m, out, rim), start, (int64_t)D->nx * D->ny * D->nz, ops) &&
+         mirror_part(D->fx, 0, largest(D->fx, 27), m.c.p) && mirror_part(D->fy, 1, largest(D->fy, 27), m.c.q) &&
+         mirror_part(D->fz, 2, largest(D->fz, 27), m.c.r);
 }
 
 template <int MODE>
@@ -527,6 +540,12 @@ static void launch_mirror(const MirrorArgs &m, const double *x, double *y, doubl
 // axis' +1) and a stress symmetric in (a, j).
 static bool mirror_fel(const cpm_fel_stencil *F, MirrorArgs &m) {
   m = MirrorArgs{};
+  m.nx = F->nx;
+  m.ny = F->ny;
+  m.nz = F->nz;
+  m.anchor = F->anchor ? 1 : 0;
+  // one plane per block would form every stress three times
+  if (!march_pays(mirror_shape(m, 87.0, 39.0), 2.5, (int64_t)m.nx * m.ny * m.nz, 312.0) || m.lx < 2) return false;
   const double big = largest(F->coef, 486);
   if (!(big > 0.0)) return false;
   const double tol = 1e-15 * big;
@@ -572,11 +591,7 @@ static bool mirror_fel(const cpm_fel_stencil *F, MirrorArgs &m) {
         else if (ax < a && std::fabs(part[ax][a][v][0] - part[a][ax][v][0]) > tol) return false;
       }
   }
-  m.nx = F->nx;
-  m.ny = F->ny;
-  m.nz = F->nz;
-  m.anchor = F->anchor ? 1 : 0;
-  return mirror_shape(m, 87.0, 39.0);
+  return true;
 }
 
 static bool grid_ok(int nx, int ny, int nz, int64_t parts) {
@@ -625,7 +640,7 @@ extern "C" int cpm_stencil_deriv(const cpm_deriv_stencil *D, const double *x, do
   }
   cudaStream_t st = (cudaStream_t)stream;
   MirrorArgs m;
-  if (mirror_deriv(D, m, mode == 0 ? 29.0 : 28.0, 1.0, mode == 0 ? kMarchDeriv : 0)) {
+  if (mode == 0 ? mirror_deriv(D, m, 29.0, 1.0, 2.5, 55.0) : mirror_deriv(D, m, 28.0, 1.0, 1.5, 79.0)) {
     if (mode == 0) launch_mirror<0>(m, x, y, alpha, -1, nullptr, stream);
     else launch_mirror<1>(m, x, y, alpha, pin, nullptr, stream);
     return check_launch("cpm_stencil_deriv");
@@ -651,7 +666,7 @@ extern "C" int cpm_stencil_strain(const cpm_deriv_stencil *D, const double *u, c
     return CPM_BAD_ARG;
   }
   MirrorArgs m;
-  if (mirror_deriv(D, m, 117.0, 3.0, kMarchDeriv)) {
+  if (mirror_deriv(D, m, 117.0, 3.0, 2.5, 186.0)) {
     launch_mirror<2>(m, u, E, 1.0, -1, R9, stream);
     return check_launch("cpm_stencil_strain");
   }
@@ -671,7 +686,7 @@ extern "C" int cpm_stencil_fel(const cpm_fel_stencil *F, const double *E0, doubl
     return CPM_BAD_ARG;
   }
   MirrorArgs m;
-  if ((int64_t)F->nx * F->ny * F->nz >= kMarchFel && mirror_fel(F, m)) {
+  if (mirror_fel(F, m)) {
     launch_mirror<3>(m, E0, b_el, 1.0, -1, nullptr, stream);
     return check_launch("cpm_stencil_fel");
   }

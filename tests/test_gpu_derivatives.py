@@ -81,3 +81,10 @@ def test_marching_scalar_product_matches_the_per_node_form(dims, nvec):
         big = float(x.abs().max())
         bound = 2 * (1e-13 * np.abs(c).max() + 54 * 2.0 ** -53 * np.abs(c).sum()) * big
         assert float((a - b).abs().max()) <= bound, name
+
+
+# grids on both sides of the rule that picks the marching form, per product: small, flat and long ones
+@pytest.mark.parametrize("dims", [(5, 7, 9), (6, 6, 7), (20, 21, 19), (44, 45, 43), (50, 45, 39), (130, 20, 33),
+                                  (9, 130, 90), (256, 4, 70), (64, 150, 5)])
+def test_products_match_on_both_sides_of_the_marching_rule(dims):
+    test_marching_products_match_the_pair_kernels(dims)
