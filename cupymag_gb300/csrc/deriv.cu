@@ -494,12 +494,13 @@ static bool march_pays(double us, double start, int64_t n, double ops) {
 // (b, c: |offset| along the others in order); false unless that is all of it, to 1e-15 of `big`.
 static bool mirror_part(const double *v, int axis, double big, double *out) {
   const double tol = 1e-15 * big;
+  if (!std::isfinite(tol)) return false;
   double sum[4] = {0, 0, 0, 0};
   for (int d = 0; d < 27; ++d) {
     const int o[3] = {d / 9 - 1, (d / 3) % 3 - 1, d % 3 - 1};
     const int e1 = o[axis == 0 ? 1 : 0] != 0, e2 = o[axis == 2 ? 1 : 2] != 0;
     if (o[axis] == 0) {
-      if (std::fabs(v[d]) > tol) return false;
+      if (!(std::fabs(v[d]) <= tol)) return false;  // (not a number fails)
     } else {
       sum[2 * e1 + e2] += o[axis] * v[d] / (2.0 * (e1 ? 2 : 1) * (e2 ? 2 : 1));
     }
@@ -507,7 +508,7 @@ static bool mirror_part(const double *v, int axis, double big, double *out) {
   for (int d = 0; d < 27; ++d) {
     const int o[3] = {d / 9 - 1, (d / 3) % 3 - 1, d % 3 - 1};
     const int e1 = o[axis == 0 ? 1 : 0] != 0, e2 = o[axis == 2 ? 1 : 2] != 0;
-    if (o[axis] != 0 && std::fabs(v[d] - o[axis] * sum[2 * e1 + e2]) > tol) return false;
+    if (o[axis] != 0 && !(std::fabs(v[d] - o[axis] * sum[2 * e1 + e2]) <= tol)) return false;
   }
   for (int e = 0; e < 4; ++e) out[e] = sum[e];
   return true;
@@ -547,7 +548,7 @@ static bool mirror_fel(const cpm_fel_stencil *F, MirrorArgs &m) {
   // one plane per block would form every stress three times
   if (!march_pays(mirror_shape(m, 87.0, 39.0), 2.5, (int64_t)m.nx * m.ny * m.nz, 312.0) || m.lx < 2) return false;
   const double big = largest(F->coef, 486);
-  if (!(big > 0.0)) return false;
+  if (!(big > 0.0) || !std::isfinite(big)) return false;
   const double tol = 1e-15 * big;
   // parts of every block: odd along one axis, even along the others
   double part[3][3][6][4];  // [axis][a][v]
@@ -569,7 +570,7 @@ static bool mirror_fel(const cpm_fel_stencil *F, MirrorArgs &m) {
           }
       }
       for (int d = 0; d < 27; ++d)
-        if (std::fabs(rest[d]) > tol) return false;
+        if (!(std::fabs(rest[d]) <= tol)) return false;
     }
   const int voigt[3][3] = {{0, 3, 5}, {3, 1, 4}, {5, 4, 2}};
   double *unit[3] = {m.c.p, m.c.q, m.c.r};
@@ -584,11 +585,11 @@ static bool mirror_fel(const cpm_fel_stencil *F, MirrorArgs &m) {
     for (int a = 0; a < 3; ++a)
       for (int v = 0; v < 6; ++v) {
         for (int e = 0; e < 4; ++e)
-          if (std::fabs(part[ax][a][v][e] - part[ax][a][v][0] * unit[ax][e]) > tol) return false;
+          if (!(std::fabs(part[ax][a][v][e] - part[ax][a][v][0] * unit[ax][e]) <= tol)) return false;
         double &c = m.C[voigt[a][ax]][v];
         if (a < ax) c = part[ax][a][v][0];                     // (a, ax) first seen from the smaller index
         else if (a == ax) c = part[ax][a][v][0];
-        else if (ax < a && std::fabs(part[ax][a][v][0] - part[a][ax][v][0]) > tol) return false;
+        else if (!(std::fabs(part[ax][a][v][0] - part[a][ax][v][0]) <= tol)) return false;
       }
   }
   return true;

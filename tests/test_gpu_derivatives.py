@@ -88,3 +88,28 @@ def test_marching_scalar_product_matches_the_per_node_form(dims, nvec):
                                   (9, 130, 90), (256, 4, 70), (64, 150, 5)])
 def test_products_match_on_both_sides_of_the_marching_rule(dims):
     test_marching_products_match_the_pair_kernels(dims)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_coefficients_that_are_not_finite_reach_the_result(bad):
+    """A coefficient outside the mirror form's pattern (dx = 0 in F_x) that is not finite is no rounding of zero: the
+    products with that stencil are not finite anywhere, on grids that otherwise march."""
+    from cupymag_gb300.core.assemble_simulation_operators import SimulationOperators
+    from cupymag_gb300.utils.stencil_derivatives import StencilCoupling, StencilDerivatives
+    from cupymag_gb300.workloads import hex_params
+    cell = SimulationOperators(hex_params(6, 1, True, True), device="cuda")
+    fx, fy, fz = (f.copy() for f in cell.stencil_derivatives().coef)
+    fel = cell.stencil_coupling().coef.copy()
+    dims = (44, 45, 43)
+    n = dims[0] * dims[1] * dims[2]
+    rng = np.random.default_rng(1)
+    dev = lambda *s: torch.as_tensor(rng.normal(size=s), device="cuda")  # noqa: E731
+    fx[12] = bad       # offset (0, 0, -1)
+    D = StencilDerivatives(*dims, fx, fy, fz)
+    H = D.hd_into(dev(n), torch.empty((n, 3), dtype=torch.float64, device="cuda"))
+    assert not torch.isfinite(H[:, 0]).any() and torch.isfinite(H[:, 1:]).all()
+    b = D.demag_rhs_into(dev(n, 3), None, torch.empty(n, dtype=torch.float64, device="cuda"), pin=0)
+    assert not torch.isfinite(b[1:]).any()
+    fel[12 * 1 + 27 * 2] = bad   # block (0, 2)
+    r = StencilCoupling(*dims, fel).spmv(dev(6 * n)).reshape(3, n)
+    assert not torch.isfinite(r[0, 1:]).any() and torch.isfinite(r[1:]).all()
