@@ -90,6 +90,7 @@ _PROTOS = {
     "cpm_cg_workspace_bytes": (C.c_size_t, [i64, C.c_int, C.c_int]),
     "cpm_cg_stencil_workspace_bytes": (C.c_size_t, [i64, C.c_int, C.c_int]),
     "cpm_cg_stencil_workspace": (C.c_size_t, [C.POINTER(Stencil), C.c_int, C.c_int]),
+    "cpm_stencil_cheb_steps": (C.c_int, [C.POINTER(Stencil), C.c_int, dbl, C.c_int]),
     "cpm_stencil_df_error_bound": (C.c_double, [C.POINTER(Stencil)]),
     "cpm_cg_solve": (C.c_int, [C.POINTER(CSR), vp, vp, C.c_int, C.POINTER(CGOpts), vp, C.c_size_t, vp, vp]),
     "cpm_cg_solve_noalloc": (C.c_int, [C.POINTER(CSR), vp, vp, C.c_int, C.POINTER(CGOpts), vp, vp]),

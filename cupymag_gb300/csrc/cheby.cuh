@@ -87,6 +87,10 @@ struct ChebSys {
   int cta0, ncta;
 };
 
+// Chunks of a pass at most, as the partials of cpm_cg_solve_stencil's workspace hold them.  Planes of more tiles
+// than that (2.36 M nodes) have no such cut: their solves keep CG.
+constexpr int64_t kChebMaxChunks = (int64_t)(kPartHalf / kChebSlot);
+
 // Partition of a system's passes: enough chunks to fill the GPU when the system runs alone, as few
 // planes of overlap as that allows.  `slots` CTAs are resident.
 inline void cheb_split(int nx, int tiles, int sms, int slots, int &lx, int &ranges) {
@@ -96,6 +100,7 @@ inline void cheb_split(int nx, int tiles, int sms, int slots, int &lx, int &rang
   for (int nr = 1; nr <= nx; ++nr) {
     const int l = (nx + nr - 1) / nr, r = (nx + l - 1) / l;
     const int64_t ch = (int64_t)tiles * r;
+    if (nr > 1 && ch > kChebMaxChunks) break;
     const int64_t ctas = ch < slots ? ch : slots, loops = (ch + ctas - 1) / ctas;
     const int64_t per_sm = (ctas + sms - 1) / sms;
     // a tile-plane costs its SM about 400 cycles of L2 traffic and a plane about 500 of latency

@@ -1027,30 +1027,38 @@ static float *cheb_vec(float *base, const cpm_stencil *s, int nrhs, int k) {
 // Bytes in front of the solvers' vectors in a workspace.
 static size_t head_bytes() { return layout(0, 1, 1, nullptr, nullptr); }
 
-// Launch of the Chebyshev solve; *done tells whether it applies: the default form, the error bound of a
-// double-float residual (and with it of an x held as two floats) at most a quarter of the tolerance, and
-// at least four times the steps of a cold start before maxiter (nearer to it CG's smaller count may decide
-// between converged and not).
+// Whether a solve runs the Chebyshev iteration, and its operator and layout: the error bound of a double-float
+// residual (and with it of an x held as two floats) at most a quarter of the tolerance, at least four times the steps
+// of a cold start before maxiter (nearer to it CG's smaller count may decide between converged and not), and planes
+// that the partials can hold (kChebMaxChunks).
+static bool cheb_rule(const cpm_stencil *s, int nrhs, double tol, int maxiter, int sms, ChebOp *op, ChebSys *y) {
+  const double e = df_error_bound(s);
+  if (!(e > 0.0 && e <= 0.25 * tol) || !cheb_operator(s->coef, s->ncomp, op) || maxiter < 4 * cheb_cold_steps(*op, tol))
+    return false;
+  op->df_err = e;
+  *y = ChebSys{};
+  y->nx = s->nx;
+  y->ny = s->ny;
+  y->nz = s->nz;
+  y->n = s->nx * s->ny * s->nz;
+  cheb_layout(*y, nrhs, sms);
+  return (size_t)y->half <= kPartHalf;
+}
+
+// Launch of the Chebyshev solve; *done tells whether it applies (cheb_rule, and a form that asks for it).
 template <int NR>
 static int launch_cheb(const cpm_stencil *s, const cpm_cg_opts *o, const StencilCG &cg, Workspace &w, float *vecs,
                        cudaStream_t st, bool *done) {
   *done = false;
   ChebSolve a;
-  const double e = df_error_bound(s);
+  ChebSys &y = a.sys;
+  const int sms = sm_count();
   if (!vecs || (o->form != CPM_CG_FORM_DEFAULT && o->form != CPM_CG_FORM_FP64_RESIDUALS) ||
-      !(e > 0.0 && e <= 0.25 * o->tol) || !cheb_operator(s->coef, s->ncomp, &a.op) ||
-      o->maxiter < 4 * cheb_cold_steps(a.op, o->tol))
+      !cheb_rule(s, NR, o->tol, o->maxiter, sms, &a.op, &y))
     return CPM_OK;
   a.cg = cg;
   a.op.df = o->form == CPM_CG_FORM_DEFAULT;
-  a.op.df_err = e;
   a.op.timeout_ns = cg.timeout_ns;
-  ChebSys &y = a.sys;
-  y = ChebSys{};
-  y.nx = s->nx;
-  y.ny = s->ny;
-  y.nz = s->nz;
-  y.n = cg.S.n;
   y.flags = s->flags;
   y.b = cg.b;
   y.x = cg.x;
@@ -1062,9 +1070,6 @@ static int launch_cheb(const cpm_stencil *s, const cpm_cg_opts *o, const Stencil
   for (int k = 0; k < 5; ++k) y.v[k] = cheb_vec(vecs, s, NR, k);
   y.part = w.part;
   y.bar = w.bar;
-  const int sms = sm_count();
-  cheb_layout(y, NR, sms);
-  if ((size_t)y.half > kPartHalf) return CPM_OK;
   int occ = 0;
   CPM_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cheb_stencil_kernel<NR>, kChebThreads, 0));
   if (occ < 1) return CPM_OK;
@@ -1218,6 +1223,15 @@ extern "C" size_t cpm_cg_stencil_workspace_bytes(int64_t unknowns, int nrhs, int
   using namespace cpm;
   const size_t base = layout(unknowns, nrhs, precision ? 1 : 0, nullptr, nullptr);
   return precision ? base + align256(sizeof(float) * (size_t)unknowns * nrhs) : base;
+}
+
+extern "C" int cpm_stencil_cheb_steps(const cpm_stencil *S, int nrhs, double tol, int maxiter) {
+  using namespace cpm;
+  if (check_stencil(S, "cpm_stencil_cheb_steps") || (nrhs != 1 && nrhs != 3)) return 0;
+  ChebOp op;
+  ChebSys y;
+  const int sms = sm_count();
+  return cheb_rule(S, nrhs, tol, maxiter, sms > 0 ? sms : 152, &op, &y) ? cheb_cold_steps(op, tol) : 0;
 }
 
 extern "C" size_t cpm_cg_stencil_workspace(const cpm_stencil *S, int nrhs, int precision) {

@@ -186,3 +186,28 @@ def test_the_default_form_runs_the_schedule(name, steps):
             assert inf["status"] == 0 and abs(inf["iters"][0] - steps) <= 1, inf
             assert inf["iters"][:nrhs] == inf["iters"][:1] * nrhs and inf["outer"] == inf["df_updates"] == 1, inf
             assert cg["iters"][0] < steps - 2, cg
+
+
+@pytest.mark.parametrize("dims,nrhs", [((672, 672, 672), 1), ((3, 1500, 1500), 3), ((1200, 330, 260), 3)])
+def test_large_grids_run_the_schedule(dims, nrhs):
+    """Grids whose residual passes are cut by what the partial sums hold, and the flattest planes: the schedule's steps
+    and the stopping test against an FP64 product."""
+    from cupymag_gb300 import _native as N
+    from cupymag_gb300.solvers.linear_solvers import CGSolver, decode_info, new_info
+    from cupymag_gb300.utils.stencil_operator import StencilOperator
+    n = dims[0] * dims[1] * dims[2]
+    free, _ = torch.cuda.mem_get_info()
+    if free < 70 * n * nrhs + (8 << 30):
+        pytest.skip("not enough device memory")
+    op = StencilOperator(*dims, _case((4, 4, 4), 0)[1]["A1"].coef_host)
+    steps = N.lib().cpm_stencil_cheb_steps(op.struct(), nrhs, TOL, 20000)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    b = torch.randn((n, 3) if nrhs == 3 else n, dtype=torch.float64, device="cuda", generator=g)
+    x, info = torch.zeros_like(b), new_info(1)
+    CGSolver().launch(op, b, x, info[0], tol=TOL, maxiter=20000, precision="IR")
+    inf = decode_info(info[0].cpu().numpy())
+    assert inf["status"] == 0 and steps == 40 and abs(inf["iters"][0] - steps) <= 1, inf
+    r = torch.linalg.norm(b - op.spmv(x), dim=0)
+    assert bool((r <= 1.001 * TOL * torch.linalg.norm(b, dim=0)).all())
+    del b, x, r
+    torch.cuda.empty_cache()

@@ -429,3 +429,44 @@ def test_flags_mark_neighbours_of_excluded_and_of_unpinned_columns():
     pin_only = np.zeros(n, dtype=np.uint8)
     pin_only[node(2, 1, 4)] = ROW_IDENTITY | COL_EXCLUDED
     assert StencilOperator(nx, ny, nz, np.ones(27), pin_only, device="cpu").anchor == node(2, 1, 4)
+
+
+def _gs_stencil(dims, coef):
+    from cupymag_gb300 import _native as N
+    s = N.Stencil()
+    s.nx, s.ny, s.nz, s.ncomp = (*dims, 1)
+    s.coef[:27] = tuple(float(v) for v in np.asarray(coef).reshape(-1))
+    s.flags = None
+    return s
+
+
+def _gs_coefs():
+    from cupymag_gb300.core.assemble_simulation_operators import SimulationOperators
+    from cupymag_gb300.physics import structured_hex as SH
+    p = G.params(G.load("hex_me_rot")).with_(Nx=8, Ny=8, Nz=8, Ndx=2, Ndy=2, Ndz=2)
+    S = SimulationOperators(p, device="cpu")
+    e = S._cell()
+    return {"A1": SH.stencil_from_element(e["K"] * S.alpha1 + e["M"]),
+            "A2": SH.stencil_from_element(e["K"] * S.alpha2 + e["M"]), "A_demag": SH.stencil_from_element(e["K"])}
+
+
+def test_chebyshev_rule_takes_grids_of_any_size():
+    """The projection operators run Chebyshev steps (40 and 60 to 1e-10) on every grid whose y-z plane the partial sums
+    can hold, cubes up to 1200^3 among them, with one and three right-hand sides; larger planes, the demag operator and
+    a maxiter below four times the steps keep CG."""
+    from cupymag_gb300 import _native as N
+    from cupymag_gb300.build import build
+    build()
+    lib = N.load()
+    coefs = _gs_coefs()
+    steps = lambda dims, name="A1", nrhs=1, tol=1e-10, maxiter=20000: lib.cpm_stencil_cheb_steps(  # noqa: E731
+        _gs_stencil(dims, coefs[name]), nrhs, tol, maxiter)
+    for nrhs in (1, 3):
+        for edge in [*range(4, 40), *range(48, 1201, 16), 997]:
+            assert steps((edge,) * 3, nrhs=nrhs) == 40, (edge, nrhs)
+        for dims in ((3, 1500, 1500), (2000, 800, 900), (5000, 400, 300), (7, 2000, 1000), (60000, 150, 150)):
+            assert steps(dims, "A2", nrhs) in (60, 61), (dims, nrhs)
+    assert steps((3, 1600, 1500)) == 0
+    assert steps((64, 64, 64), "A_demag") == 0
+    assert steps((64, 64, 64), maxiter=159) == 0 and steps((64, 64, 64), maxiter=160) == 40
+    assert steps((64, 64, 64), tol=1e-12) == 0
