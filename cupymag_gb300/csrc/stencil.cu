@@ -1010,11 +1010,12 @@ bool cheb_operator(const double *c, int ncomp, ChebOp *op) {
 
 int cheb_cold_steps(const ChebOp &op, double tol) {
   int steps = 0;
-  for (double res = 1.0; res > kChebAim * tol && steps < 100000;) {
+  double res = 1.0;
+  do {  // one cycle at least, however loose the tolerance
     const int k = cheb_steps(res, kChebAim * tol, op.acosh_s);
     steps += k;
     res *= std::max(2.0 * std::exp(-k * op.acosh_s), 1.0 / kChebCycle);
-  }
+  } while (res > kChebAim * tol && steps < 100000);
   return steps;
 }
 

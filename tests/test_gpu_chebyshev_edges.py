@@ -211,3 +211,16 @@ def test_large_grids_run_the_schedule(dims, nrhs):
     assert bool((r <= 1.001 * TOL * torch.linalg.norm(b, dim=0)).all())
     del b, x, r
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("maxiter", [0, 1, 2, 5])
+@pytest.mark.parametrize("tol", [0.5, 1.9, 2.0, 40.0])
+def test_loose_tolerances_respect_a_small_maxiter(tol, maxiter):
+    """A tolerance that x = 0 meets already, with fewer iterations allowed than four cycles: CG's record (one
+    iteration at least)."""
+    from cupymag_gb300 import _native as N
+    op = _case((8, 7, 9), 2)[1]["A1"]
+    b = np.random.default_rng(3).normal(size=op.n)
+    _, inf = _solve(op, b, tol=tol, maxiter=maxiter)
+    _, cg = _solve(op, b, tol=tol, maxiter=maxiter, form=N.CG_FORM_THREE_BARRIER)
+    assert inf["iters"][0] <= max(maxiter, 1) and inf["status"] == cg["status"] and inf["iters"] == cg["iters"], (inf, cg)
