@@ -904,7 +904,7 @@ static StencilOp to_op(const cpm_stencil *s) {
 }
 
 // The quad form needs whole quads in every z-line and 4-byte aligned flags
-// (the solver's own vectors are 256-byte aligned).
+// (the solver's own vectors lie at multiples of 256 bytes from the workspace's start).
 static bool quads_ok(const cpm_stencil *s) {
   return (s->nz & 3) == 0 && ((uintptr_t)s->flags & 3) == 0;
 }
@@ -1135,7 +1135,7 @@ static int launch_stencil_cg(const cpm_stencil *s, const double *b, double *x, c
   if (fp64 && NC == 3) a.even = even3_coefs(s->coef, a.e64, kEvenRounding);
   if constexpr (NC == 1) {
     if (!fp64) {
-      a.quads = quads_ok(s) && ((uintptr_t)x & 15) == 0 ? 1 : 0;
+      a.quads = quads_ok(s) && (((uintptr_t)x | (uintptr_t)w.bar) & 15) == 0 ? 1 : 0;
       bool done;
       if (int err = launch_cheb<NR>(s, o, a, w, vecs, st, &done)) return err;
       if (done) return CPM_OK;
@@ -1151,8 +1151,8 @@ static int launch_stencil_cg(const cpm_stencil *s, const double *b, double *x, c
     return CPM_CUDA_ERROR;
   }
   const int64_t n = a.S.n;
-  // vector quads need whole quads per z-line, aligned flags and an aligned x
-  a.quads = quads_ok(s) && ((uintptr_t)x & 15) == 0 ? 1 : 0;
+  // vector quads need whole quads per z-line, aligned flags and an aligned x and workspace
+  a.quads = quads_ok(s) && (((uintptr_t)x | (uintptr_t)w.bar) & 15) == 0 ? 1 : 0;
   // The FP32 quad product (4 outputs and 27 independent loads per thread) runs best on few, full
   // CTAs.  The elastic per-DOF product (grids with nz % 4 != 0) needs every resident CTA to hide its
   // gather latency; the scalar ones do not.  Measured on GB300: elastic 81^3 per DOF 80 us per
@@ -1205,9 +1205,10 @@ extern "C" int cpm_cg_solve_stencil(const cpm_stencil *S, const double *b, doubl
   float *xlo = nullptr;
   if (prec && workspace_bytes >= cpm_cg_stencil_workspace_bytes(unknowns, nrhs, prec))
     xlo = (float *)((char *)workspace + need);
-  // the Chebyshev iteration's vectors take the place of the CG's where they fit
+  // the Chebyshev iteration's vectors take the place of the CG's where they fit; its quads need 16-byte alignment
+  // for every nz, so other workspaces keep CG
   float *vecs = nullptr;
-  if (prec && workspace_bytes >= cpm_cg_stencil_workspace(S, nrhs, prec))
+  if (prec && ((uintptr_t)workspace & 15) == 0 && workspace_bytes >= cpm_cg_stencil_workspace(S, nrhs, prec))
     vecs = (float *)((char *)workspace + head_bytes());
   cudaStream_t st = (cudaStream_t)stream;
   if (S->ncomp == 3) return launch_stencil_cg<3, 1>(S, b, x, opts, w, xlo, vecs, info_dev, st);

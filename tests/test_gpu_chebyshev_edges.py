@@ -224,3 +224,33 @@ def test_loose_tolerances_respect_a_small_maxiter(tol, maxiter):
     _, inf = _solve(op, b, tol=tol, maxiter=maxiter)
     _, cg = _solve(op, b, tol=tol, maxiter=maxiter, form=N.CG_FORM_THREE_BARRIER)
     assert inf["iters"][0] <= max(maxiter, 1) and inf["status"] == cg["status"] and inf["iters"] == cg["iters"], (inf, cg)
+
+
+@pytest.mark.parametrize("nrhs", [1, 3])
+@pytest.mark.parametrize("nz", [7, 8])
+def test_workspaces_aligned_to_8_bytes_are_solved(nz, nrhs):
+    """A workspace of the full size that starts 8 bytes off a 16-byte boundary runs CG on scalar loads (it is compared
+    with the aligned one only in what both promise: status, stopping test and pinned rows)."""
+    import ctypes as C
+    from cupymag_gb300 import _native as N
+    from cupymag_gb300.solvers.linear_solvers import decode_info, new_info
+    S, so, csr = _case((9, 8, nz), 2)
+    A, op = csr["A1"], so["A1"]
+    b = np.random.default_rng(nz).normal(size=(op.n, 3) if nrhs == 3 else op.n)
+    bd = torch.as_tensor(b, device="cuda").contiguous()
+    L = N.lib()
+    nbytes = int(L.cpm_cg_stencil_workspace(op.struct(), nrhs, 1))
+    mem = torch.zeros(nbytes + 64, dtype=torch.uint8, device="cuda")
+    for off in (0, 8):
+        ws = mem[off:off + nbytes]
+        assert ws.data_ptr() % 16 == off
+        x, info = torch.zeros_like(bd), new_info(1)
+        o = N.CGOpts()
+        o.tol, o.maxiter, o.precision, o.inner_tol, o.barrier_timeout_s = TOL, 20000, 1, 1e-5, 2.0
+        assert L.cpm_cg_solve_stencil(op.struct(), bd.data_ptr(), x.data_ptr(), nrhs, C.byref(o), ws.data_ptr(), nbytes,
+                                      info[0].data_ptr(), N.stream_ptr()) == N.CPM_OK
+        inf = decode_info(info[0].cpu().numpy())
+        assert inf["status"] == 0 and (inf["iters"][0] >= 39) == (off == 0), inf
+        xs = x.cpu().numpy()
+        assert max(_residuals(A, b, xs)) <= TOL
+        assert np.array_equal(xs[S.DefDOF], b[S.DefDOF])
