@@ -1046,6 +1046,22 @@ static bool cheb_rule(const cpm_stencil *s, int nrhs, double tol, int maxiter, i
   return (size_t)y->half <= kPartHalf;
 }
 
+// Solves of one right-hand side on short z-lines, which the padding to multiples of 8 floats doubles (nz = 3, 4, 8) or
+// lengthens by a third (12, 16, 24), and which CG takes in aligned quads: from a cold start that the host knows of CG
+// is faster there, for nz = 4 on large planes from any start.  Measured on GB300, us per solve, CG / Chebyshev, cold
+// A1 and A2: 100x100x8 230, 254 / 218, 309; 256x256x3 287, 355 / 342, 481; 256x256x8 287, 365 / 326, 452; 600x600x4
+// 613, 728 / 736, 957 (warm 453 / 509); 600x600x8 680, 830 / 932, 1259 (warm 889 / 583); 64x64x16 226, 249 / 197,
+// 279; 128x128x24 285, 361 / 286, 407; 600x600x12 1144, 1184 / 1085, 1477; 1000x1000x12 2511, 3256 / 2779, 3792;
+// 600x600x32 2385, 3094 / 2273, 3228; 600x600x9 1442, 1502 / 1098, 1509.
+static bool cheb_thin(const ChebSys &y, const ChebOp &op, int nrhs, bool cold) {
+  if (nrhs != 1 || (y.nz != 3 && (y.nz & 3))) return false;
+  if (y.nz == 4 && y.n >= 1000000) return true;
+  const double pad = (double)y.pitch / y.nz;
+  if (!cold || y.n < 30000) return false;
+  // 1.3: from 4 M nodes on, or with more than 50 steps to 1e-10 (A2 but not A1)
+  return pad >= 2.0 || (pad >= 1.3 && (y.n >= 4000000 || cheb_cold_steps(op, 1e-10) > 50));
+}
+
 // Launch of the Chebyshev solve; *done tells whether it applies (cheb_rule, and a form that asks for it).
 template <int NR>
 static int launch_cheb(const cpm_stencil *s, const cpm_cg_opts *o, const StencilCG &cg, Workspace &w, float *vecs,
@@ -1055,7 +1071,8 @@ static int launch_cheb(const cpm_stencil *s, const cpm_cg_opts *o, const Stencil
   ChebSys &y = a.sys;
   const int sms = sm_count();
   if (!vecs || (o->form != CPM_CG_FORM_DEFAULT && o->form != CPM_CG_FORM_FP64_RESIDUALS) ||
-      !cheb_rule(s, NR, o->tol, o->maxiter, sms, &a.op, &y))
+      !cheb_rule(s, NR, o->tol, o->maxiter, sms, &a.op, &y) ||
+      cheb_thin(y, a.op, NR, !o->use_init_dev && !o->use_init_host))
     return CPM_OK;
   a.cg = cg;
   a.op.df = o->form == CPM_CG_FORM_DEFAULT;

@@ -209,7 +209,9 @@ size_t cpm_cg_stencil_workspace_bytes(int64_t unknowns, int nrhs, int precision)
 size_t cpm_cg_stencil_workspace(const cpm_stencil *S, int nrhs, int precision);
 /* The rule behind that, on the host: the steps of a cold solve to tol where cpm_cg_solve_stencil (precision 1, form
  * DEFAULT, that workspace) runs the Chebyshev iteration, 0 where it runs CG.  Besides the operator, the tolerance and
- * maxiter the rule looks at the grid: y-z planes of more than 2.36 million nodes keep CG. */
+ * maxiter the rule looks at the grid: y-z planes of more than 2.36 million nodes keep CG.  (Beyond it, solves of one
+ * right-hand side on large grids of nz = 3, 4, 8, 12, 16 or 24 that start from zero on the host's word keep CG, which
+ * is faster on such short lines.) */
 int cpm_stencil_cheb_steps(const cpm_stencil *S, int nrhs, double tol, int maxiter);
 /* The bound behind that choice, as a multiple of ||b||: 2 g sum|c| / sigma_min with g = 128 * 2^-48 and
  * sigma_min a lower bound of the stencil's symbol (its part even along every axis is minimised over the 8

@@ -254,3 +254,22 @@ def test_workspaces_aligned_to_8_bytes_are_solved(nz, nrhs):
         xs = x.cpu().numpy()
         assert max(_residuals(A, b, xs)) <= TOL
         assert np.array_equal(xs[S.DefDOF], b[S.DefDOF])
+
+
+@pytest.mark.parametrize("dims,name", [((120, 100, 3), "A1"), ((130, 80, 4), "A2"), ((90, 60, 8), "A1"),
+                                       ((500, 800, 12), "A1"), ((60, 50, 16), "A2")])
+def test_cold_solves_of_one_vector_on_short_lines_keep_cg(dims, name):
+    """One right-hand side from a cold start runs CG on grids of short z-lines, three right-hand sides and warm starts
+    (nz = 4 below a million nodes) the Chebyshev schedule; both meet the stopping test."""
+    from cupymag_gb300.utils.stencil_operator import StencilOperator
+    op = StencilOperator(*dims, _case((4, 4, 4), 0)[1][name].coef_host)
+    rng = np.random.default_rng(dims[2])
+    b = rng.normal(size=(op.n, 3))
+    one = np.ascontiguousarray(b[:, 0])
+    product = lambda v: op.spmv(torch.as_tensor(v, device="cuda")).cpu().numpy()  # noqa: E731
+    for rhs, x0, cheb in ((one, None, False), (b, None, True), (one, rng.normal(size=op.n), True)):
+        x, inf = _solve(op, rhs, x0)
+        _, cg = _solve(op, rhs, x0, form=1)
+        assert inf["status"] == 0 and (inf["iters"] != cg["iters"]) == cheb, (inf, cg)
+        r = np.linalg.norm((rhs - product(x)).reshape(op.n, -1), axis=0)
+        assert np.all(r <= 1.001 * TOL * np.linalg.norm(rhs.reshape(op.n, -1), axis=0))
