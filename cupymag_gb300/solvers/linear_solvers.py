@@ -38,15 +38,20 @@ class CGSolver:
         # residual is FP64)
         self.df_residual = True
 
-    def workspace(self, n, nrhs, prec, stencil=None):
-        """Device workspace of a solve; stencil operators (`stencil`: the operator) take the size that enables
-        every form."""
-        key = (n, nrhs, prec, None if stencil is None else (stencil.nx, stencil.ny, stencil.nz))
+    def workspace(self, n, nrhs, prec, stencil=False):
+        """Device workspace of a solve.  stencil: the operator of a stencil solve (the size that enables every form),
+        True for a stencil solve of n unknowns on an unknown grid (every form of CG), False for a CSR solve."""
+        grid = (stencil.nx, stencil.ny, stencil.nz) if hasattr(stencil, "ncomp") else bool(stencil)
+        key = (n, nrhs, prec, grid)
         ws = self._ws.get(key)
         if ws is None:
             L = N.lib()
-            nbytes = L.cpm_cg_workspace_bytes(n, nrhs, prec) if stencil is None else \
-                L.cpm_cg_stencil_workspace(stencil.struct(), nrhs, prec)
+            if grid is False:
+                nbytes = L.cpm_cg_workspace_bytes(n, nrhs, prec)
+            elif grid is True:
+                nbytes = L.cpm_cg_stencil_workspace_bytes(n, nrhs, prec)
+            else:
+                nbytes = L.cpm_cg_stencil_workspace(stencil.struct(), nrhs, prec)
             ws = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
             self._ws[key] = ws
         return ws
@@ -79,7 +84,7 @@ class CGSolver:
         if not (b.is_contiguous() and x.is_contiguous()) or b.dtype != torch.float64 or x.dtype != torch.float64:
             raise TypeError("b and x must be contiguous float64 device tensors")
         stencil = hasattr(A, "ncomp")
-        ws = self.workspace(n, nrhs, prec, stencil=A if stencil else None)
+        ws = self.workspace(n, nrhs, prec, stencil=A if stencil else False)
         o = N.CGOpts()
         o.tol = float(tol)
         o.maxiter = int(maxiter)

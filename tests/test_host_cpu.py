@@ -470,3 +470,24 @@ def test_chebyshev_rule_takes_grids_of_any_size():
     assert steps((64, 64, 64), "A_demag") == 0
     assert steps((64, 64, 64), maxiter=159) == 0 and steps((64, 64, 64), maxiter=160) == 40
     assert steps((64, 64, 64), tol=1e-12) == 0
+
+
+def test_solver_workspaces_by_kind():
+    """CGSolver.workspace takes a flag (CSR or stencil) or the stencil operator, and keeps one buffer per kind."""
+    from cupymag_gb300 import _native as N
+    from cupymag_gb300.build import build
+    from cupymag_gb300.solvers.linear_solvers import CGSolver
+    from cupymag_gb300.utils.stencil_operator import StencilOperator
+    import torch
+    build()
+    lib = N.load()
+    solver = CGSolver(device=torch.device("cpu"))
+    op = StencilOperator(8, 9, 10, _gs_coefs()["A1"], device="cpu")
+    n = op.n
+    for nrhs, prec in ((1, 0), (3, 0), (1, 1), (3, 1)):
+        sizes = [lib.cpm_cg_workspace_bytes(n, nrhs, prec), lib.cpm_cg_stencil_workspace_bytes(n, nrhs, prec),
+                 lib.cpm_cg_stencil_workspace(op.struct(), nrhs, prec)]
+        kinds = (False, True, op)
+        assert [solver.workspace(n, nrhs, prec, stencil=k).numel() for k in kinds] == sizes
+        assert solver.workspace(n, nrhs, prec).numel() == sizes[0]
+        assert all(solver.workspace(n, nrhs, prec, k) is solver.workspace(n, nrhs, prec, stencil=k) for k in kinds)
