@@ -100,6 +100,7 @@ _PROTOS = {
                                        vp]),
     "cpm_batch_work_bytes": (i64, [i32, i32, i32, i32, i32, i32]),
     "cpm_batch_plan_bytes": (C.c_int, [C.POINTER(BatchSystem), i32, i32, i32, i32, C.POINTER(i64)]),
+    "cpm_batch_plan_bytes_for": (C.c_int, [C.POINTER(BatchSystem), i32, i32, i32, i32, vp, C.POINTER(i64)]),
     "cpm_batch_plan_build": (C.c_int, [C.POINTER(BatchSystem), i32, i32, i32, i32, vp, vp, i64, C.POINTER(BatchPlan),
                                        vp]),
     "cpm_cg_solve_blockdiag": (C.c_int, [C.POINTER(BatchPlan), C.POINTER(CGOpts), vp]),

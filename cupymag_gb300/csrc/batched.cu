@@ -998,12 +998,30 @@ static size_t cheb_sys_bytes(const cpm_batch_system &y, int nrhs, int sms) {
 
 static int cheb_max_grid() { return sm_count() * kChebBlocks; }
 
+// Whether a plan's systems may run Chebyshev steps, by the single solver's rule: the operator (its factors to *op, the
+// residual's error bound to *err; coef NULL: not known, taken to fit), then each system's tolerance and maxiter.
+static bool cheb_plan_fits(const double *coef, ChebOp *op, double *err) {
+  if (!coef) return true;
+  cpm_stencil one{};
+  one.ncomp = 1;
+  for (int i = 0; i < 27; ++i) one.coef[i] = coef[i];
+  *err = df_error_bound(&one);
+  return *err > 0.0 && cheb_operator(coef, 1, op);
+}
+static bool cheb_system_fits(const cpm_batch_system &y, const double *coef, const ChebOp &op, double err) {
+  return !coef || (err <= 0.25 * y.tol && y.maxiter >= 4 * cheb_cold_steps(op, y.tol));
+}
+
 // Bytes of the Chebyshev part (0 where the plan has none).
-static size_t cheb_part_bytes(const cpm_batch_system *sys, int nsys, int ncomp, int nrhs, int precision) {
-  if (ncomp != 1 || !precision || nsys > cheb_max_grid()) return 0;
-  size_t b = cheb_plan_layout(0, nsys, cheb_max_grid()).total;
-  for (int s = 0; s < nsys; ++s) b += cheb_sys_bytes(sys[s], nrhs, sm_count());
-  return b;
+static size_t cheb_part_bytes(const cpm_batch_system *sys, int nsys, int ncomp, int nrhs, int precision,
+                              const double *coef) {
+  ChebOp op;
+  double err = 0.0;
+  if (ncomp != 1 || !precision || nsys > cheb_max_grid() || !cheb_plan_fits(coef, &op, &err)) return 0;
+  size_t b = 0;
+  for (int s = 0; s < nsys; ++s)
+    if (cheb_system_fits(sys[s], coef, op, err)) b += cheb_sys_bytes(sys[s], nrhs, sm_count());
+  return b ? b + cheb_plan_layout(0, nsys, cheb_max_grid()).total : 0;
 }
 
 struct Assignment {
@@ -1093,7 +1111,21 @@ extern "C" int cpm_batch_plan_bytes(const cpm_batch_system *sys, int32_t nsys, i
     return CPM_BAD_ARG;
   }
   *bytes = (int64_t)(plan_layout(A.total_chunks, nsys, A.grid).total +
-                     cheb_part_bytes(sys, nsys, ncomp, nrhs, precision));
+                     cheb_part_bytes(sys, nsys, ncomp, nrhs, precision, nullptr));
+  return CPM_OK;
+}
+
+extern "C" int cpm_batch_plan_bytes_for(const cpm_batch_system *sys, int32_t nsys, int32_t ncomp, int32_t nrhs,
+                                        int32_t precision, const double *coef, int64_t *bytes) {
+  using namespace cpm;
+  Assignment A;
+  if (int e = assign(sys, nsys, ncomp, nrhs, precision, A, "cpm_batch_plan_bytes_for")) return e;
+  if (!coef || !bytes) {
+    set_error("cpm_batch_plan_bytes_for: coef or bytes is NULL");
+    return CPM_BAD_ARG;
+  }
+  *bytes = (int64_t)(plan_layout(A.total_chunks, nsys, A.grid).total +
+                     cheb_part_bytes(sys, nsys, ncomp, nrhs, precision, coef));
   return CPM_OK;
 }
 
@@ -1104,12 +1136,14 @@ extern "C" int cpm_batch_plan_build(const cpm_batch_system *sys, int32_t nsys, i
   Assignment A;
   if (int e = assign(sys, nsys, ncomp, nrhs, precision, A, "cpm_batch_plan_build")) return e;
   const PlanLayout L = plan_layout(A.total_chunks, nsys, A.grid);
-  const size_t total = L.total + cheb_part_bytes(sys, nsys, ncomp, nrhs, precision);
-  if (!coef || !plan || !plan_dev || plan_bytes < (int64_t)total || ((uintptr_t)plan_dev & 255)) {
+  if (!coef || !plan || !plan_dev || plan_bytes < (int64_t)L.total || ((uintptr_t)plan_dev & 255)) {
     set_error("cpm_batch_plan_build: bad arguments (coef, plan and a 256-byte aligned device buffer of at least "
-              "%zu bytes)", total);
+              "%zu bytes)", L.total);
     return CPM_BAD_ARG;
   }
+  // the Chebyshev part where the operator takes it and the buffer holds it
+  size_t total = L.total + cheb_part_bytes(sys, nsys, ncomp, nrhs, precision, coef);
+  if (plan_bytes < (int64_t)total) total = L.total;
   std::vector<BSeg> segs(nsys);
   std::vector<int> cmap(A.grid);
   int chunk0 = 0, cta0 = 0;
@@ -1161,20 +1195,16 @@ extern "C" int cpm_batch_plan_build(const cpm_batch_system *sys, int32_t nsys, i
   std::vector<int> cseg, ccta;
   ChebLayout CL{};
   if (total > L.total) {
-    // the systems that the single solver would run with Chebyshev steps, by the same rule
-    cpm_stencil one{};
-    one.ncomp = 1;
-    for (int i = 0; i < 27; ++i) one.coef[i] = coef[i];
     ChebOp op;
-    const double e = df_error_bound(&one);
-    if (e > 0.0 && cheb_operator(coef, 1, &op)) {
+    double e;
+    if (cheb_plan_fits(coef, &op, &e)) {
       const int sms = sm_count(), gmax = cheb_max_grid();
       int64_t work = 0;
       CL = cheb_plan_layout(L.total, nsys, gmax);
       size_t at = CL.total;
       for (int s = 0; s < nsys; ++s) {
         const cpm_batch_system &y = sys[s];
-        if (!(e <= 0.25 * y.tol) || y.maxiter < 4 * cheb_cold_steps(op, y.tol)) continue;
+        if (!cheb_system_fits(y, coef, op, e)) continue;
         ChebSys S{};
         S.nx = y.nx;
         S.ny = y.ny;

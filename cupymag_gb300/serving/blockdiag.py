@@ -76,14 +76,14 @@ class BlockDiagPlan:
             e.info, e.work = s.info.data_ptr(), s.work.data_ptr()
         L = N.lib()
         nbytes = N.i64()
-        N.check(L.cpm_batch_plan_bytes(arr, len(systems), ncomp, nrhs, self.precision, C.byref(nbytes)),
-                "cpm_batch_plan_bytes")
+        coef = (C.c_double * 243)()
+        coef[:op0.coef_host.size] = tuple(float(v) for v in op0.coef_host)
+        N.check(L.cpm_batch_plan_bytes_for(arr, len(systems), ncomp, nrhs, self.precision, coef, C.byref(nbytes)),
+                "cpm_batch_plan_bytes_for")
         dev = device or systems[0].b.device
         self.mem = torch.empty(int(nbytes.value), dtype=torch.uint8, device=dev)
         if self.mem.data_ptr() % 256:
             raise RuntimeError("plan memory is not 256-byte aligned")
-        coef = (C.c_double * 243)()
-        coef[:op0.coef_host.size] = tuple(float(v) for v in op0.coef_host)
         self.plan = N.BatchPlan()
         N.check(L.cpm_batch_plan_build(arr, len(systems), ncomp, nrhs, self.precision, coef, self.mem.data_ptr(),
                                        nbytes.value, C.byref(self.plan), N.stream_ptr()), "cpm_batch_plan_build")

@@ -68,9 +68,9 @@ def estimate_bytes(p, precision="IR") -> int:
     cheb = 0
     if precision != "DP":
         # Chebyshev solves: five FP32 vectors of padded z-lines per right-hand side of the projection plans (3, 1, 1
-        # and 3) and, in small runs, of the demag plan
+        # and 3)
         pitch = (int(p.Nz) + 9) // 8 * 8
-        cheb = 5 * 4 * int(p.Nx) * int(p.Ny) * pitch * (8 if n >= FFT_MIN_DOFS else 9)
+        cheb = 5 * 4 * int(p.Nx) * int(p.Ny) * pitch * 8
     return int((per * n + cheb) * 1.05) + (8 << 20)
 
 

@@ -253,12 +253,16 @@ typedef struct {
 /* Work-vector bytes of one system on an nx x ny x nz grid; 0 for invalid dimensions. */
 int64_t cpm_batch_work_bytes(int32_t nx, int32_t ny, int32_t nz, int32_t ncomp, int32_t nrhs, int32_t precision);
 
-/* Device bytes of the plan for these systems (CTA assignment, partial sums, tables). */
+/* Device bytes of the plan for these systems (CTA assignment, partial sums, tables, and the Chebyshev vectors of
+ * scalar systems in precision 1), for any operator.  cpm_batch_plan_bytes_for: for the operator of these
+ * coefficients (host, 27*ncomp*ncomp), without the vectors where it cannot run Chebyshev steps. */
 int cpm_batch_plan_bytes(const cpm_batch_system *sys, int32_t nsys, int32_t ncomp, int32_t nrhs,
                          int32_t precision, int64_t *bytes);
+int cpm_batch_plan_bytes_for(const cpm_batch_system *sys, int32_t nsys, int32_t ncomp, int32_t nrhs,
+                             int32_t precision, const double *coef, int64_t *bytes);
 
 /* Build the plan into plan_dev (256-byte aligned, plan_bytes from
- * cpm_batch_plan_bytes): copies the system table to the device and waits for
+ * either query; a plan without room for the Chebyshev vectors runs CG): copies the system table to the device and waits for
  * the copy on `stream`, so it is called outside stream capture, once per
  * batch composition.  coef: host, 27*ncomp*ncomp FP64 coefficients. */
 int cpm_batch_plan_build(const cpm_batch_system *sys, int32_t nsys, int32_t ncomp, int32_t nrhs,

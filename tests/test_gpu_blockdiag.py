@@ -149,3 +149,51 @@ def test_blockdiag_two_barrier_form_alone_equals_in_mix(kind):
         assert mix[i][1]["status"] == 0, mix[i][1]
         r = b - A @ mix[i][0]
         assert np.all(np.linalg.norm(r, axis=0) <= 1e-10 * np.linalg.norm(b, axis=0) * 1.001), (kind, i)
+
+
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_plans_reserve_chebyshev_vectors_only_where_they_can_run(nrhs):
+    """The plan memory of the demag operator, of FP64 plans and of systems whose maxiter rules Chebyshev steps out has
+    no room for their vectors; a projection plan has five padded vectors, and one built into less memory runs CG and
+    meets the stopping test."""
+    import ctypes as C
+    from cupymag_gb300 import _native as N
+    from cupymag_gb300.core.assemble_simulation_operators import SimulationOperators
+    from cupymag_gb300.serving.blockdiag import BlockDiagPlan, BlockSystem, work_bytes
+    from cupymag_gb300.solvers.linear_solvers import decode_info, new_info
+    from . import _golden as G
+    dims = (20, 18, 22)
+    p = G.params(G.load("hex_me_rot")).with_(Nx=dims[0], Ny=dims[1], Nz=dims[2], Ndx=2, Ndy=2, Ndz=2)
+    S = SimulationOperators(p)
+    so, csr = S.stencil_operators(), S.host_operators()
+    rng = np.random.default_rng(4)
+
+    def system(name, prec, maxiter):
+        op = so[name]
+        b = torch.as_tensor(rng.normal(size=(op.n, 3) if nrhs == 3 else op.n), device="cuda")
+        work = torch.empty(work_bytes(dims, 1, nrhs, prec), dtype=torch.uint8, device="cuda")
+        return BlockSystem(op, b, torch.zeros_like(b), new_info(1)[0], work, 1e-10, maxiter)
+
+    vectors = 5 * 4 * nrhs * dims[0] * dims[1] * 24
+    for name, prec, maxiter, has in (("A1", "IR", 20000, True), ("A1", "IR", 100, False), ("A1", "DP", 20000, False),
+                                     ("A_demag", "IR", 20000, False)):
+        plan = BlockDiagPlan([system(name, prec, maxiter)], prec)
+        assert (plan.mem.numel() >= vectors) == has and (plan.plan.cheb_nsys == 1) == has, (name, prec, maxiter)
+        full = plan if has and prec == "IR" else None
+        if full is not None:
+            small = plan.mem.numel() - vectors
+            arr, s = (N.BatchSystem * 1)(), plan.systems[0]
+            e = arr[0]
+            e.nx, e.ny, e.nz = dims
+            e.maxiter, e.tol, e.flags = s.maxiter, s.tol, s.op.flags.data_ptr()
+            e.b, e.x, e.info, e.work = s.b.data_ptr(), s.x.data_ptr(), s.info.data_ptr(), s.work.data_ptr()
+            coef = (C.c_double * 243)()
+            coef[:27] = tuple(float(v) for v in s.op.coef_host)
+            N.check(N.lib().cpm_batch_plan_build(arr, 1, 1, nrhs, 1, coef, plan.mem.data_ptr(), small,
+                                                 C.byref(plan.plan), N.stream_ptr()), "cpm_batch_plan_build")
+            assert plan.plan.cheb_nsys == 0
+            plan.launch()
+            assert decode_info(s.info.cpu().numpy())["status"] == 0
+            b, x = (t.cpu().numpy().reshape(s.op.n, -1) for t in (s.b, s.x))
+            r = np.linalg.norm(b - csr[name] @ x, axis=0)
+            assert np.all(r <= 1e-10 * np.linalg.norm(b, axis=0))
