@@ -239,6 +239,18 @@ inline bool even8_coefs(const double *coef, double *c8) {
   return true;
 }
 
+// A row without flags of a scalar stencil, for one vector, all loads before the sum (scalar_rows' order): left to
+// itself the compiler keeps as few loads in flight as its register count allows.
+__device__ __forceinline__ double plain_row(const StencilOp &S, const double *x, int dof) {
+  const Nbr b = neighbours(S, dof);
+  double v[27], y = 0.0;
+#pragma unroll
+  for (int d = 0; d < 27; ++d) v[d] = x[b.xi[d / 9] + b.yj[(d / 3) % 3] + b.zk[d % 3]];
+#pragma unroll
+  for (int d = 0; d < 27; ++d) y = fma(S.c64[d], v[d], y);
+  return y;
+}
+
 // A row with flags f of such a march, for right-hand side r (the rows of apply_c): excluded columns are read as zeros,
 // so all 27 loads are in flight at once (a march takes its flagged rows one after the other), and one right-hand side
 // is formed, not all.  Mass matrix with a defect on GB300, us per product, apply_c / this: three vectors 20^3
