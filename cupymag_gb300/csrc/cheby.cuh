@@ -432,8 +432,9 @@ __device__ __forceinline__ void cheb_put(float *p, int k, int nz, float v) {
 // the chunk partials of |r|^2 per right-hand side, of the unrounded r in FP64 (the stopping test is on this norm);
 // b times `down` where that is set.  Every value enters renormalised (h + l = hi + lo exactly, |lo| <= 2^-24 |hi|).  In units of 2^-48 of the sum of the terms'
 // magnitudes: the z and y sums of a term are within 8 (df_add: 3 per sum, twice, and 2 for the dropped
-// renormalisation), its product within 13 (df::fma), and the 4 + 4 accumulations and two sums of planes
-// within 3 each: 57, inside the 94 that the bound of df_error_bound allows.
+// renormalisation), its product within 13 (df::fma), the 4 + 4 accumulations and two sums of planes within 3 each; the
+// difference from b adds 3 and b's split 2, as |b| is at most that sum and |r|: 56, inside the 94 that the bound of
+// df_error_bound allows.
 template <int NR>
 __device__ __forceinline__ void cheb_residual(const ChebSys &S, const ChebOp &op, int l, const double *down,
                                               const float *h, const float *lo, float *r, double *half,
